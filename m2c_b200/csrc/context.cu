@@ -150,7 +150,8 @@ struct m2cg_ctx {
   // tensor maps of the stage inputs: [0..1] the step state in the compute
   // type (Vf[b] mixed, V[b] FP64), [2..3] P[b]
   CUtensorMap tmap[4];
-  bool tma_ok = false;       // maps built (else the kernel copies values one by one)
+  CUtensorMap tid;           // material IDs
+  int tile_y = 8;            // rows per stage tile
   int cur = 0;
   uint8_t* id = nullptr;
   // mesh
@@ -160,6 +161,7 @@ struct m2cg_ctx {
   int* lK[3] = {};
   double* lC[3] = {};
   int ntx = 1, nty = 1, nitems = 1;
+  StageVariant variant = {};
   std::vector<double> hdx, hdy, hdz, hxc, hyc, hzc;
   // device scratch: clock [t, dt, tmax, cfl], dtmin bits, flags, error
   double* clock = nullptr;
@@ -190,42 +192,40 @@ struct m2cg_ctx {
 // driver entry point, so the library links only the CUDA runtime) of the
 // stage kernel's plane input: 4D (x, y, z, component) over one
 // five-component buffer, box = one plane of a tile with its halo,
-// STAGE_TMA_BX x (TY + 4) x 1 x 5 elements. Out-of-range x/y cells read as
-// zero; the kernel rebuilds them by the boundary rule.
-static m2cg_status encode_stage_map(m2cg_ctx* c, CUtensorMap* m, const void* base, bool f32, int ty) {
-  static PFN_cuTensorMapEncodeTiled encode = nullptr;
-  if (!encode) {
+// STAGE_TMA_BX x (TY + 4) x 1 x 5 elements; and 3D over the material IDs,
+// box STAGE_TMA_IX x (TY + 4) x 1. Out-of-range x/y cells read as zero; the
+// kernel rebuilds them by the boundary rule.
+static m2cg_status encode_stage_map(m2cg_ctx* c, CUtensorMap* m, void* base, CUtensorMapDataType type, size_t es,
+                                    cuuint32_t bx, int ty) {
+  static const PFN_cuTensorMapEncodeTiled encode = [] {  // looked up once: a look-up takes milliseconds
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn)
-      return fail(M2CG_ERR_CUDA, "cuTensorMapEncodeTiled not available from the driver");
-    encode = (PFN_cuTensorMapEncodeTiled)fn;
-  }
-  const size_t es = f32 ? 4 : 8;
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return (PFN_cuTensorMapEncodeTiled)fn;
+  }();
+  if (!encode) return fail(M2CG_ERR_CUDA, "cuTensorMapEncodeTiled not available from the driver");
+  const cuuint32_t rank = es == 1 ? 3 : 4;
   cuuint64_t dims[4] = {(cuuint64_t)c->nx, (cuuint64_t)c->ny, (cuuint64_t)c->nz, 5};
   cuuint64_t strides[3] = {(cuuint64_t)(c->px * es), (cuuint64_t)(c->plane * es), (cuuint64_t)(c->cstride * es)};
-  cuuint32_t box[4] = {(cuuint32_t)STAGE_TMA_BX, (cuuint32_t)(ty + 4), 1, 5};
+  cuuint32_t box[4] = {bx, (cuuint32_t)(ty + 4), 1, 5};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = encode(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
-                      const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  CUresult r = encode(m, type, rank, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(M2CG_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   return M2CG_OK;
 }
 
-// A map that cannot be encoded leaves tma_ok false: the stage kernel then
-// copies plane values one by one.
 static m2cg_status make_stage_tensor_maps(m2cg_ctx* c) {
   const bool mixed = c->scheme.precision == M2CG_PREC_MIXED;
-  const int ty = mixed ? StageTY<float, false>::value : StageTY<double, false>::value;
-  for (int b = 0; b < 2; b++) {
-    m2cg_status st = encode_stage_map(c, &c->tmap[b], mixed ? c->blk[3][b] : c->blk[0][b], mixed, ty);
-    if (!st) st = encode_stage_map(c, &c->tmap[2 + b], c->blk[2][b], mixed, ty);
-    if (st) return st;  // the stage kernel then copies plane values one by one
+  const CUtensorMapDataType type = mixed ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+  m2cg_status st = encode_stage_map(c, &c->tid, c->id, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, STAGE_TMA_IX, c->tile_y);
+  for (int b = 0; b < 2 && !st; b++) {
+    st = encode_stage_map(c, &c->tmap[b], mixed ? c->blk[3][b] : c->blk[0][b], type, mixed ? 4 : 8, STAGE_TMA_BX, c->tile_y);
+    if (!st) st = encode_stage_map(c, &c->tmap[2 + b], c->blk[2][b], type, mixed ? 4 : 8, STAGE_TMA_BX, c->tile_y);
   }
-  c->tma_ok = true;
-  return M2CG_OK;
+  return st;
 }
 
 static double* dalloc(size_t n, m2cg_status* st) {
@@ -319,7 +319,7 @@ static MatParams to_params(const m2cg_material& m) {
   return p;
 }
 
-static void set_stage_items(m2cg_ctx* c, bool multi);
+static m2cg_status set_stage_items(m2cg_ctx* c);
 
 extern "C" m2cg_status m2cg_create(const m2cg_grid* grid, const m2cg_scheme* scheme, const m2cg_material* mats,
                                    int nmat, const m2cg_levelset* ls, int nls, m2cg_ctx** out) {
@@ -378,8 +378,9 @@ extern "C" m2cg_status m2cg_create(const m2cg_grid* grid, const m2cg_scheme* sch
       }
     }
   }
-  if (!st) make_stage_tensor_maps(c);
   if (cudaMalloc((void**)&c->id, c->nalloc) != cudaSuccess) st = fail(M2CG_ERR_NOMEM, "cudaMalloc id failed");
+  c->tile_y = mixed ? StageShape<float>::ty : StageShape<double>::ty;
+  if (!st) st = make_stage_tensor_maps(c);
   if (!st) cudaMemsetAsync(c->id, 0, c->nalloc, c->stream);
   axis_mesh(grid->nx, grid->x0, grid->xmax, grid->xc, grid->dx, c->hxc, c->hdx);
   axis_mesh(grid->ny, grid->y0, grid->ymax, grid->yc, grid->dy, c->hyc, c->hdy);
@@ -403,6 +404,7 @@ extern "C" m2cg_status m2cg_create(const m2cg_grid* grid, const m2cg_scheme* sch
     c->g.lu[a] = uni && !A.empty() ? 1 : 0;
     if (!A.empty()) {
       c->g.lA0[a] = A[0]; c->g.lB0[a] = B[0]; c->g.lK0[a] = K[0]; c->g.lC0[a] = Cm[0];
+      c->g.fA0[a] = (float)A[0]; c->g.fB0[a] = (float)B[0]; c->g.fC0[a] = (float)Cm[0];
     }
     upload_vec(&c->lA[a], A, c->stream, &st);
     upload_vec(&c->lB[a], B, c->stream, &st);
@@ -444,10 +446,6 @@ extern "C" m2cg_status m2cg_create(const m2cg_grid* grid, const m2cg_scheme* sch
     sk.ed[m] = make_eos<double>(p);
     sk.ef[m] = make_eos<float>(p);
   }
-  size_t smem = scheme->precision == M2CG_PREC_MIXED ? stage_smem_mixed(nls == 1) : stage_smem_fp64(nls == 1);
-  int maxsm = 0;
-  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  if (!st && (size_t)maxsm < smem) st = fail(M2CG_ERR_CUDA, "stage kernel needs %zu B shared memory, device has %d", smem, maxsm);
   if (!st && nls == 1) {
     const double* xc[3] = {c->hxc.data(), c->hyc.data(), c->hzc.data()};
     const double* dxs[3] = {c->hdx.data(), c->hdy.data(), c->hdz.data()};
@@ -460,19 +458,13 @@ extern "C" m2cg_status m2cg_create(const m2cg_grid* grid, const m2cg_scheme* sch
     st = viscous_create(c->stream, g, sk.ed, mats, nmat, xc, dxs, &c->visc);
     if (st) fail(st, "viscous-flux buffers could not be allocated");
   }
+  c->ntx = (c->nx + TX - 1) / TX;
+  c->nty = (c->ny + c->tile_y - 1) / c->tile_y;
+  if (!st) st = set_stage_items(c);
   if (st) {
     m2cg_destroy(c);
     return st;
   }
-  // The (x,y) tiles x z planes are shared evenly by a persistent grid of
-  // resident CTAs, each share at least 8 planes long (the plane pipeline's
-  // prologue costs about 2.5 planes per segment).
-  const int ty = scheme->precision == M2CG_PREC_MIXED
-                     ? StageTY<float, false>::value
-                     : (nls == 1 ? StageTY<double, true>::value : StageTY<double, false>::value);
-  c->ntx = (c->nx + TX - 1) / TX;
-  c->nty = (c->ny + ty - 1) / ty;
-  set_stage_items(c, nls == 1);
   CK(cudaStreamSynchronize(c->stream));
   *out = c;
   return M2CG_OK;
@@ -825,13 +817,22 @@ static void rk_coeffs(int r, int s, double& a_prev, double& a_un, double& b) {
   a_prev = 2.0 / 3.0; a_un = 1.0 / 3.0; b = 2.0 / 3.0;
 }
 
-// Persistent grid size of the stage kernel variant (two-material or not).
-static void set_stage_items(m2cg_ctx* c, bool multi) {
-  const int resident = c->scheme.precision == M2CG_PREC_MIXED ? stage_resident_mixed(c->scheme.flux, multi)
-                                                               : stage_resident_fp64(c->scheme.flux, multi);
-  const long long units = (long long)c->ntx * c->nty * c->nz;
-  const long long by_len = (units + 7) / 8;
-  c->nitems = (int)std::max<long long>(1, std::min<long long>(resident, by_len));
+// The stage kernel variant in use and its persistent grid: the (x,y) tiles x
+// z planes are shared evenly by resident CTAs.
+static m2cg_status set_stage_items(m2cg_ctx* c) {
+  StageVariant& v = c->variant;
+  v.flux = c->scheme.flux;
+  v.multi = c->mp != nullptr || c->walls != nullptr;  // the two-material kernel also carries the branch of cut faces
+  v.walls = c->walls != nullptr;
+  v.cons = c->sk.rec_var != 0 && c->sk.rec_linear;
+  v.sg = true;
+  for (const m2cg_material& m : c->mats) v.sg = v.sg && m.eos == M2CG_EOS_SG;
+  int resident = 1;
+  const cudaError_t e = c->scheme.precision == M2CG_PREC_MIXED ? prepare_stage_mixed(v, &resident)
+                                                                : prepare_stage_fp64(v, &resident);
+  if (e != cudaSuccess) return fail(M2CG_ERR_CUDA, "stage kernel set-up: %s", cudaGetErrorString(e));
+  c->nitems = (int)std::min<long long>(resident, (long long)c->ntx * c->nty * c->nz);
+  return M2CG_OK;
 }
 
 extern "C" m2cg_status m2cg_set_wall_faces(m2cg_ctx* c, int n, const int* faces, const double* nwall_fwd,
@@ -842,8 +843,7 @@ extern "C" m2cg_status m2cg_set_wall_faces(m2cg_ctx* c, int n, const int* faces,
   if (n == 0) {
     walls_destroy(c->walls);
     c->walls = nullptr;
-    set_stage_items(c, c->mp != nullptr);
-    return M2CG_OK;
+    return set_stage_items(c);
   }
   // HeatDiffusionOperator::AddDiffusionFluxes leaves cut faces alone (its
   // EBDS argument is unused); ViscosityOperator's ghost-fluid population at
@@ -851,10 +851,6 @@ extern "C" m2cg_status m2cg_set_wall_faces(m2cg_ctx* c, int n, const int* faces,
   if (viscous_has_viscosity(c->visc))
     return fail(M2CG_ERR_UNSUPPORTED,
                 "cut faces with viscous materials (the viscosity operator's ghost-fluid branch) are not implemented");
-  const size_t smem = c->scheme.precision == M2CG_PREC_MIXED ? stage_smem_mixed(true) : stage_smem_fp64(true);
-  int maxsm = 0;
-  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  if ((size_t)maxsm < smem) return fail(M2CG_ERR_CUDA, "stage kernel needs %zu B shared memory, device has %d", smem, maxsm);
   Walls* w = nullptr;
   char msg[200] = {0};
   const m2cg_status st = walls_create(c->stream, c->g, c->nalloc, c->scheme, n, faces, nwall_fwd, uwall_fwd, nwall_bwd,
@@ -862,25 +858,21 @@ extern "C" m2cg_status m2cg_set_wall_faces(m2cg_ctx* c, int n, const int* faces,
   if (st) return fail(st, "cut faces refused: %s", msg);
   walls_destroy(c->walls);
   c->walls = w;
-  set_stage_items(c, true);
-  return M2CG_OK;
+  return set_stage_items(c);
 }
 
 static m2cg_status launch_stage(m2cg_ctx* c, StageArgs& a) {
   a.ntx = c->ntx;
   a.nty = c->nty;
   a.nitems = c->nitems;
-  int grid = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c->profile) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, c->stream);
   }
-  // the two-material kernel variant also carries the branch of cut faces
-  const bool multi = c->mp != nullptr || c->walls != nullptr;
-  cudaError_t e = c->scheme.precision == M2CG_PREC_MIXED ? launch_stage_mixed(a, c->stream, multi, &grid)
-                                                          : launch_stage_fp64(a, c->stream, multi, &grid);
+  cudaError_t e = c->scheme.precision == M2CG_PREC_MIXED ? launch_stage_mixed(a, c->variant, c->stream)
+                                                          : launch_stage_fp64(a, c->variant, c->stream);
   if (c->profile) {
     cudaEventRecord(e1, c->stream);
     c->ev.push_back(e0);
@@ -893,7 +885,7 @@ static m2cg_status launch_stage(m2cg_ctx* c, StageArgs& a) {
 
 static void base_args(m2cg_ctx* c, StageArgs& a) {
   memset(&a, 0, sizeof a);
-  a.use_tma = c->tma_ok && c->g.bc[0] != BC_PERIODIC && c->g.bc[2] != BC_PERIODIC;
+  a.tid = c->tid;
   a.g = c->g;
   a.s = c->sk;
   a.id = c->id;

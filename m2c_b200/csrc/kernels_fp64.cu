@@ -5,15 +5,12 @@
 
 namespace m2c {
 
-size_t stage_smem_fp64(bool multi) {
-  return multi ? sizeof(StageSmemAll<double, StageTY<double, true>::value, true>)
-               : sizeof(StageSmemAll<double, StageTY<double, false>::value, false>);
+cudaError_t launch_stage_fp64(const StageArgs& a, const StageVariant& v, cudaStream_t s) {
+  return stage_variant<double>(v, &a, s, nullptr);
 }
 
-cudaError_t launch_stage_fp64(const StageArgs& a, cudaStream_t s, bool multi, int* grid_out) {
-  return launch_stage_t<double>(a, s, multi, grid_out);
+cudaError_t prepare_stage_fp64(const StageVariant& v, int* resident) {
+  return stage_variant<double>(v, nullptr, nullptr, resident);
 }
-
-int stage_resident_fp64(int flux, bool multi) { return blocks_per_sm_t<double>(flux, multi); }
 
 }  // namespace m2c

@@ -7,15 +7,12 @@
 
 namespace m2c {
 
-size_t stage_smem_mixed(bool multi) {
-  return multi ? sizeof(StageSmemAll<float, StageTY<float, true>::value, true>)
-               : sizeof(StageSmemAll<float, StageTY<float, false>::value, false>);
+cudaError_t launch_stage_mixed(const StageArgs& a, const StageVariant& v, cudaStream_t s) {
+  return stage_variant<float>(v, &a, s, nullptr);
 }
 
-cudaError_t launch_stage_mixed(const StageArgs& a, cudaStream_t s, bool multi, int* grid_out) {
-  return launch_stage_t<float>(a, s, multi, grid_out);
+cudaError_t prepare_stage_mixed(const StageVariant& v, int* resident) {
+  return stage_variant<float>(v, nullptr, nullptr, resident);
 }
-
-int stage_resident_mixed(int flux, bool multi) { return blocks_per_sm_t<float>(flux, multi); }
 
 }  // namespace m2c

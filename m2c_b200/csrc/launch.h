@@ -9,90 +9,66 @@
 
 namespace m2c {
 
-constexpr int STAGE_TY = 8;
-#ifndef M2C_STAGE_TY_F32
-#define M2C_STAGE_TY_F32 16
-#endif
-// Tile height per instantiation: 32 x 8 for the FP64 kernels, 32 x 16 for
-// the FP32 (mixed) kernels.
-template <typename T, bool MULTI> struct StageTY { static constexpr int value = STAGE_TY; };
-template <bool MULTI> struct StageTY<float, MULTI> { static constexpr int value = M2C_STAGE_TY_F32; };
+// The kernel variant of a stage: two materials (or cut faces), non-primitive
+// reconstruction, faces cut by an embedded surface, stiffened gases only.
+struct StageVariant {
+  int flux;
+  bool multi, cons, walls, sg;
+};
 
-size_t stage_smem_fp64(bool multi);
-size_t stage_smem_mixed(bool multi);
-// Launch one stage on a persistent grid of min(nitems, SMs x resident CTAs
-// per SM) CTAs sharing the work evenly. *grid_out reports the grid.
-cudaError_t launch_stage_fp64(const StageArgs& a, cudaStream_t s, bool multi, int* grid_out);
-cudaError_t launch_stage_mixed(const StageArgs& a, cudaStream_t s, bool multi, int* grid_out);
-// Resident CTAs on the whole device of the stage kernel for (flux, multi);
-// each precision's translation unit instantiates only its own kernels.
-int stage_resident_fp64(int flux, bool multi);
-int stage_resident_mixed(int flux, bool multi);
+// Launch one stage on a persistent grid of a.nitems CTAs sharing the work
+// evenly; the variant was prepared.
+cudaError_t launch_stage_fp64(const StageArgs& a, const StageVariant& v, cudaStream_t s);
+cudaError_t launch_stage_mixed(const StageArgs& a, const StageVariant& v, cudaStream_t s);
+// Make the variant launchable on the current device (its shared memory) and
+// report the CTAs of it that the device holds at once.
+cudaError_t prepare_stage_fp64(const StageVariant& v, int* resident);
+cudaError_t prepare_stage_mixed(const StageVariant& v, int* resident);
 
-template <typename T, int FLUX, bool MULTI, bool CONS = false, bool WALLS = false>
-cudaError_t stage_occupancy(int* per_sm, int* nsm) {
-  constexpr int TY = StageTY<T, MULTI>::value;
-  auto k = stage_kernel<T, TY, FLUX, MULTI, CONS, WALLS>;
-  const size_t smem = sizeof(StageSmemAll<T, TY, MULTI>);
+template <typename T, int FLUX, bool MULTI, bool CONS, bool WALLS, bool SG>
+cudaError_t stage_one(const StageArgs* a, cudaStream_t s, int* resident) {
+  auto k = stage_kernel<T, FLUX, MULTI, CONS, WALLS, SG>;
+  const size_t smem = sizeof(StageSmem<T, StageShape<T>::ty, MULTI>);
+  const dim3 block(TX, StageShape<T>::warps);
+  if (a) {
+    k<<<a->nitems, block, smem, s>>>(*a);
+    return cudaGetLastError();
+  }
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  e = cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, TX * TY, smem);
-  if (*per_sm < 1) *per_sm = 1;
+  int dev = 0, nsm = 0, per_sm = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block.x * block.y, smem);
+  if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
+  *resident = per_sm * nsm;
   return e;
 }
 
-template <typename T, int FLUX, bool MULTI, bool CONS, bool WALLS = false>
-cudaError_t launch_stage_one(const StageArgs& a, cudaStream_t s, int* grid_out) {
-  constexpr int TY = StageTY<T, MULTI>::value;
-  auto k = stage_kernel<T, TY, FLUX, MULTI, CONS, WALLS>;
-  const size_t smem = sizeof(StageSmemAll<T, TY, MULTI>);
-  int per_sm = 1, nsm = 148;
-  cudaError_t e = stage_occupancy<T, FLUX, MULTI, CONS, WALLS>(&per_sm, &nsm);
-  if (e != cudaSuccess) return e;
-  int grid = a.nitems < per_sm * nsm ? a.nitems : per_sm * nsm;
-  if (grid_out) *grid_out = grid;
-  k<<<grid, dim3(TX, TY), smem, s>>>(a);
-  return cudaGetLastError();
-}
-
 template <typename T, int FLUX>
-cudaError_t launch_stage_f(const StageArgs& a, cudaStream_t s, bool multi, int* g) {
-  const bool cons = a.s.rec_var != 0 && a.s.rec_linear;
-  if (multi && a.wall.mask)  // faces cut by an embedded surface attached
-    return cons ? launch_stage_one<T, FLUX, true, true, true>(a, s, g)
-                : launch_stage_one<T, FLUX, true, false, true>(a, s, g);
-  if (multi)
-    return cons ? launch_stage_one<T, FLUX, true, true>(a, s, g) : launch_stage_one<T, FLUX, true, false>(a, s, g);
-  return cons ? launch_stage_one<T, FLUX, false, true>(a, s, g) : launch_stage_one<T, FLUX, false, false>(a, s, g);
+cudaError_t stage_flux(const StageVariant& v, const StageArgs* a, cudaStream_t s, int* r) {
+  if (v.cons) {  // compiled for any equation of state
+    if (v.walls) return stage_one<T, FLUX, true, true, true, false>(a, s, r);
+    return v.multi ? stage_one<T, FLUX, true, true, false, false>(a, s, r)
+                   : stage_one<T, FLUX, false, true, false, false>(a, s, r);
+  }
+  if (v.walls)
+    return v.sg ? stage_one<T, FLUX, true, false, true, true>(a, s, r)
+                : stage_one<T, FLUX, true, false, true, false>(a, s, r);
+  if (v.multi)
+    return v.sg ? stage_one<T, FLUX, true, false, false, true>(a, s, r)
+                : stage_one<T, FLUX, true, false, false, false>(a, s, r);
+  return v.sg ? stage_one<T, FLUX, false, false, false, true>(a, s, r)
+              : stage_one<T, FLUX, false, false, false, false>(a, s, r);
 }
 
+// a: launch it; NULL: prepare the variant.
 template <typename T>
-cudaError_t launch_stage_t(const StageArgs& a, cudaStream_t s, bool multi, int* g) {
-  switch (a.s.flux) {
-    case FLUX_ROE: return launch_stage_f<T, FLUX_ROE>(a, s, multi, g);
-    case FLUX_LLF: return launch_stage_f<T, FLUX_LLF>(a, s, multi, g);
-    default: return launch_stage_f<T, FLUX_HLLC>(a, s, multi, g);
+cudaError_t stage_variant(const StageVariant& v, const StageArgs* a, cudaStream_t s, int* r) {
+  switch (v.flux) {
+    case FLUX_ROE: return stage_flux<T, FLUX_ROE>(v, a, s, r);
+    case FLUX_LLF: return stage_flux<T, FLUX_LLF>(v, a, s, r);
+    default: return stage_flux<T, FLUX_HLLC>(v, a, s, r);
   }
-}
-
-template <typename T>
-int blocks_per_sm_t(int flux, bool multi) {
-  int per_sm = 1, nsm = 148;
-  switch (flux) {
-    case FLUX_ROE:
-      multi ? stage_occupancy<T, FLUX_ROE, true>(&per_sm, &nsm) : stage_occupancy<T, FLUX_ROE, false>(&per_sm, &nsm);
-      break;
-    case FLUX_LLF:
-      multi ? stage_occupancy<T, FLUX_LLF, true>(&per_sm, &nsm) : stage_occupancy<T, FLUX_LLF, false>(&per_sm, &nsm);
-      break;
-    default:
-      multi ? stage_occupancy<T, FLUX_HLLC, true>(&per_sm, &nsm) : stage_occupancy<T, FLUX_HLLC, false>(&per_sm, &nsm);
-  }
-  return per_sm * nsm;
 }
 
 }  // namespace m2c

@@ -56,6 +56,32 @@ template <typename T> M2C_HD bool finite_(T x) { return isfinite(x); }
 template <typename T> M2C_HD T pick3(int d, T a, T b, T c) { return d == 0 ? a : (d == 1 ? b : c); }
 template <typename T> M2C_HD T vnorm(int d, const T* V) { return pick3(d, V[1], V[2], V[3]); }
 
+// The FP32 build contracts products and sums into FMAs, and which ones decides
+// the last bit. These flags fix the choice where it otherwise depends on what
+// the compiler knows at a call, so that a face's flux keeps its value wherever
+// it is formed: PIN_MOMENTUM the momentum components of the physical flux (the
+// normal one fused, a tangential one rounded before it is used),
+// PIN_SOUND the stiffened gas' sound speed, PIN_ENTHALPY the kinetic energy in
+// the enthalpy, PIN_SUPERSONIC the normal momentum flux of HLLC's supersonic
+// branches (not fused). FP64 is not contracted: no effect.
+enum { PIN_MOMENTUM = 1, PIN_SOUND = 2, PIN_ENTHALPY = 4, PIN_SUPERSONIC = 8 };
+
+// a*b rounded, and a*b + c: one rounding where the FP32 build contracts, two in FP64.
+template <typename T>
+M2C_HD T mul_rounded(T a, T b) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (sizeof(T) == 4) return __fmul_rn(a, b);
+#endif
+  return a * b;
+}
+template <typename T>
+M2C_HD T mul_add(T a, T b, T c) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (sizeof(T) == 4) return __fmaf_rn(a, b, c);
+#endif
+  return a * b + c;
+}
+
 // Material parameters in arithmetic type T.
 template <typename T>
 struct Eos {
@@ -86,15 +112,25 @@ struct Eos {
     return gam1 / (T(1) - b * rho);
   }
   // VarFcnBase::ComputeSoundSpeedSquare: recomputes p from (rho, e).
-  M2C_HD T c2(T rho, T e) const { return dpdrho(rho, e) + pressure(rho, e) / rho * big_gamma(rho, e); }
-  // true = violates hyperbolicity (VarFcnSG::CheckState / VarFcnNASG::CheckState)
+  template <int PIN = 0>
+  M2C_HD T c2(T rho, T e) const {
+#if defined(__CUDA_ARCH__)
+    if constexpr ((PIN & PIN_SOUND) && sizeof(T) == 4) {
+      if (kind == EOS_SG) {
+        const T p = __fmaf_rn(__fmul_rn(gam1, rho), e, -gam_ps);
+        return __fmaf_rn(p / rho, gam1, __fmul_rn(gam1, e));
+      }
+    }
+#endif
+    return dpdrho(rho, e) + pressure(rho, e) / rho * big_gamma(rho, e);
+  }
+  // true = violates hyperbolicity (VarFcnSG::CheckState / VarFcnNASG::CheckState);
+  // one expression without short cuts, so that no branch is compiled
   M2C_HD bool bad(T rho, T p) const {
-    if (!finite_(rho) || !finite_(p)) return true;
-    return rho <= T(0) || p + pstiff <= T(0);
+    return !((fabs(rho) < T(INFINITY)) & (fabs(p) < T(INFINITY)) & (rho > T(0)) & (p + pstiff > T(0)));
   }
   M2C_HD bool bad(const T* V) const {
-    if (!finite_(V[0]) || !finite_(V[1]) || !finite_(V[2]) || !finite_(V[3]) || !finite_(V[4])) return true;
-    return bad(V[0], V[4]);
+    return !((fabs(V[1]) < T(INFINITY)) & (fabs(V[2]) < T(INFINITY)) & (fabs(V[3]) < T(INFINITY))) | bad(V[0], V[4]);
   }
   // VarFcnBase::ClipDensityAndPressure (without the U update); returns clipped?
   M2C_HD bool clip(T* V) const {
@@ -107,11 +143,24 @@ struct Eos {
   }
   // Would clip() change V? (used where the reference reverts instead)
   M2C_HD bool needs_clip(const T* V) const {
-    return V[0] < rhomin || V[4] < pmin || V[0] > rhomax || V[4] > pmax;
+    return (V[0] < rhomin) | (V[4] < pmin) | (V[0] > rhomax) | (V[4] > pmax);
+  }
+  // Both face states v - s/2 and v + s/2 physical and within the clip bounds:
+  // the smaller and the larger of the two values of a component are
+  // v -+ |s|/2, rounded alike, so one test serves both sides.
+  M2C_HD bool both_fine(const T* v, const T* s) const {
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 5; c++) ok = ok & (fabs(v[c]) + T(0.5) * fabs(s[c]) < T(INFINITY));
+    const T rl = v[0] - T(0.5) * fabs(s[0]), rh = v[0] + T(0.5) * fabs(s[0]);
+    const T pl = v[4] - T(0.5) * fabs(s[4]), ph = v[4] + T(0.5) * fabs(s[4]);
+    return ok & (rl > T(0)) & (pl + pstiff > T(0)) & (rl >= rhomin) & (pl >= pmin) & (rh <= rhomax) & (ph <= pmax);
   }
   // H = e + |u|^2/2 + p/rho (VarFcnBase::ComputeTotalEnthalpyPerUnitMass)
+  template <int PIN = 0>
   M2C_HD T enthalpy(const T* V) const {
     T e = energy(V[0], V[4]);
+    if (PIN & PIN_ENTHALPY) return mul_add(T(0.5), V[1] * V[1] + V[2] * V[2] + V[3] * V[3], e) + V[4] / V[0];
     return e + T(0.5) * (V[1] * V[1] + V[2] * V[2] + V[3] * V[3]) + V[4] / V[0];
   }
   M2C_HD void c2p(const T* U, T* V) const {
@@ -234,6 +283,59 @@ M2C_HD T limited_slope_c(int limiter, T A, T B, int k, T alpha, T dql, T dqr) {
   return T(0.5) * (dql + dqr);
 }
 
+// The five components' slopes at once: the same values as limited_slope_c of
+// each, with the limiter chosen once and no branch per component (the early
+// returns of the scalar forms cost 50 instructions a component in the stage
+// kernel, this 13). van Albada with k = 2, every uniform axis' exponent: a
+// component without a slope divides by 1, and a warp none of whose lanes has
+// one skips the divisions.
+template <typename T>
+M2C_HD void limited_slopes(int limiter, T A, T B, int k, T alpha, const T* dl, const T* dr, T* s) {
+  if (limiter == LIM_VANALBADA && k == 2) {
+    bool on[5], any = false;
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      const T q = mul_rounded(dl[c], dr[c]);
+      on[c] = !(q <= T(0)) && !(fabs(q) < T(1e-16));
+      any = any || on[c];
+      s[c] = T(0);
+    }
+    if (any) {
+#pragma unroll
+      for (int c = 0; c < 5; c++) {
+        const T p0 = mul_rounded(dl[c], dl[c]), p1 = mul_rounded(dr[c], dr[c]);
+        const T num = mul_rounded(B, mul_add(dr[c], p0, mul_rounded(dl[c], p1)));
+        const T q = num / (on[c] ? mul_add(A, p1, p0) : T(1));
+        s[c] = on[c] ? q : T(0);
+      }
+    }
+  } else if (limiter == LIM_GENMINMOD) {
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      const T a = alpha * dl[c], b = B * (dl[c] + dr[c]), d = alpha * dr[c];
+      const bool pos = dl[c] > T(0) && dr[c] > T(0), neg = dl[c] < T(0) && dr[c] < T(0);
+      T lo, hi;
+#if defined(__CUDA_ARCH__)
+      if constexpr (sizeof(T) == 4) {
+        lo = fminf(a, fminf(b, d));
+        hi = fmaxf(a, fmaxf(b, d));
+      } else
+#endif
+      {
+        lo = smin(a, smin(b, d));
+        hi = smax(a, smax(b, d));
+      }
+      s[c] = pos ? lo : (neg ? hi : T(0));
+    }
+  } else if (limiter == LIM_VANALBADA) {
+#pragma unroll
+    for (int c = 0; c < 5; c++) s[c] = lim_vanalbada(A, B, k, dl[c], dr[c]);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 5; c++) s[c] = T(0.5) * (dl[c] + dr[c]);
+  }
+}
+
 template <typename T>
 M2C_HD T limited_slope(int limiter, T A, T B, int k, T alpha, T dql, T dqr) {
   if (limiter == LIM_GENMINMOD) return lim_genminmod(A, B, alpha, dql, dqr);
@@ -343,15 +445,24 @@ M2C_HD void char_to_prim(const CharBasis<T>& b, const T* V0, const T* dW, T* dV)
 // ---------------------------------------------------------------------------
 // Physical flux in direction d (0 x / F, 1 y / G, 2 z / H).
 // ---------------------------------------------------------------------------
-template <typename T>
+template <int PIN = 0, typename T>
 M2C_HD void phys_flux(const Eos<T>& eos, int d, const T* V, T* F) {
-  T H = eos.enthalpy(V);
+  T H = eos.template enthalpy<PIN>(V);
   T vn = vnorm(d, V);
   T rvn = V[0] * vn;
   F[0] = rvn;
-  F[1] = d == 0 ? rvn * V[1] + V[4] : rvn * V[1];
-  F[2] = d == 1 ? rvn * V[2] + V[4] : rvn * V[2];
-  F[3] = d == 2 ? rvn * V[3] + V[4] : rvn * V[3];
+#if defined(__CUDA_ARCH__)
+  if constexpr ((PIN & PIN_MOMENTUM) && sizeof(T) == 4) {
+    F[1] = d == 0 ? __fmaf_rn(rvn, V[1], V[4]) : __fmul_rn(rvn, V[1]);
+    F[2] = d == 1 ? __fmaf_rn(rvn, V[2], V[4]) : __fmul_rn(rvn, V[2]);
+    F[3] = d == 2 ? __fmaf_rn(rvn, V[3], V[4]) : __fmul_rn(rvn, V[3]);
+  } else
+#endif
+  {
+    F[1] = d == 0 ? rvn * V[1] + V[4] : rvn * V[1];
+    F[2] = d == 1 ? rvn * V[2] + V[4] : rvn * V[2];
+    F[3] = d == 2 ? rvn * V[3] + V[4] : rvn * V[3];
+  }
   F[4] = rvn * H;
 }
 
@@ -400,8 +511,22 @@ M2C_HD void roe_hat(const Eos<T>& eos, int d, const T* Vm, const T* Vp, RoeHat<T
   }
 }
 
-// HLLC star-region flux F* for one side (FluxFcnHLLC.h:159-195).
+// The normal momentum flux of phys_flux with its product rounded before the
+// pressure is added (FP32, see PIN_MOMENTUM).
 template <typename T>
+M2C_HD void split_normal(int d, const T* V, T* F) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (sizeof(T) == 4) {
+    const T f = __fadd_rn(__fmul_rn(F[0], vnorm(d, V)), V[4]);
+    if (d == 0) F[1] = f;
+    else if (d == 1) F[2] = f;
+    else F[3] = f;
+  }
+#endif
+}
+
+// HLLC star-region flux F* for one side (FluxFcnHLLC.h:159-195).
+template <int PIN, typename T>
 M2C_HD void hllc_fstar(const Eos<T>& eos, int d, const T* V, T S, T Sstar, T* F) {
   T velo = vnorm(d, V);
   T rhostar = V[0] * (S - velo) / (S - Sstar);
@@ -414,19 +539,58 @@ M2C_HD void hllc_fstar(const Eos<T>& eos, int d, const T* V, T S, T Sstar, T* F)
   Us[3] = d == 2 ? Sstar : V[3];
   Us[4] = U[4] / V[0] + (Sstar - velo) * (Sstar + V[4] / (V[0] * (S - velo)));
   for (int i = 0; i < 5; i++) Us[i] = Us[i] * rhostar;
-  phys_flux(eos, d, V, F);
+  phys_flux<PIN>(eos, d, V, F);
   for (int i = 0; i < 5; i++) F[i] = F[i] + S * (Us[i] - U[i]);
 }
 
+// HLLC in FP64: the side whose state (or star state) lies at xi = 0 is chosen
+// first and evaluated once, for every lane alike, where a branch per side
+// would run both. The values are those of the general form below.
+M2C_HD int flux_hllc_one_side(const Eos<double>& eos, int d, const double* Vm, const double* Vp, double* F) {
+  RoeHat<double> h;
+  roe_hat(eos, d, Vm, Vp, h);
+  const double c2m = eos.c2(Vm[0], h.em), c2p = eos.c2(Vp[0], h.ep);
+  if (c2m < 0.0 || c2p < 0.0) return ERR_SOUND;
+  const double cm = sqrt(c2m), cp = sqrt(c2p);
+  const double vm = vnorm(d, Vm), vp = vnorm(d, Vp);
+  const double u_hat = roe_avg(h.sm, vm, h.sp, vp);
+  const double Sm = smin(vm - cm, u_hat - h.c_hat), Sp = smax(vp + cp, u_hat + h.c_hat);
+  const bool allm = 0.0 <= Sm, allp = !allm && 0.0 >= Sp, star = !allm && !allp;
+  const double Sstar = (Vp[4] - Vm[4] + Vm[0] * vm * (Sm - vm) - Vp[0] * vp * (Sp - vp)) /
+                       (star ? Vm[0] * (Sm - vm) - Vp[0] * (Sp - vp) : 1.0);
+  if (star && !(Sstar >= 0.0) && !(Sstar <= 0.0)) return ERR_HLLC;
+  const bool left = allm || (star && Sstar >= 0.0);
+  double V[5];
+#pragma unroll
+  for (int i = 0; i < 5; i++) V[i] = left ? Vm[i] : Vp[i];
+  const double e = left ? h.em : h.ep, vn = left ? vm : vp, S = left ? Sm : Sp;
+  const double ek = e + 0.5 * (V[1] * V[1] + V[2] * V[2] + V[3] * V[3]);
+  const double H = ek + V[4] / V[0], rvn = V[0] * vn;
+  F[0] = rvn;
+#pragma unroll
+  for (int i = 0; i < 3; i++) F[1 + i] = d == i ? rvn * V[1 + i] + V[4] : rvn * V[1 + i];
+  F[4] = rvn * H;
+  if (star) {
+    const double rhostar = V[0] * (S - vn) / (S - Sstar), U4 = V[0] * ek;
+    const double E = U4 / V[0] + (Sstar - vn) * (Sstar + V[4] / (V[0] * (S - vn)));
+    F[0] = F[0] + S * (rhostar - V[0]);
+#pragma unroll
+    for (int i = 0; i < 3; i++) F[1 + i] = F[1 + i] + S * ((d == i ? Sstar : V[1 + i]) * rhostar - V[0] * V[1 + i]);
+    F[4] = F[4] + S * (E * rhostar - U4);
+  }
+  return ERR_NONE;
+}
+
 // Returns an error code (ERR_NONE on success).
-template <typename T>
+template <int PIN = 0, typename T>
 M2C_HD int flux_hllc(const Eos<T>& eos, int d, const T* Vm, const T* Vp, T* F) {
+  if constexpr (sizeof(T) == 8) return flux_hllc_one_side(eos, d, Vm, Vp, F);
   RoeHat<T> h;
   roe_hat(eos, d, Vm, Vp, h);
-  T cm = eos.c2(Vm[0], h.em);
+  T cm = eos.template c2<PIN>(Vm[0], h.em);
   if (cm < T(0)) return ERR_SOUND;
   cm = sqrt(cm);
-  T cp = eos.c2(Vp[0], h.ep);
+  T cp = eos.template c2<PIN>(Vp[0], h.ep);
   if (cp < T(0)) return ERR_SOUND;
   cp = sqrt(cp);
   T vm = vnorm(d, Vm), vp = vnorm(d, Vp);
@@ -434,16 +598,18 @@ M2C_HD int flux_hllc(const Eos<T>& eos, int d, const T* Vm, const T* Vp, T* F) {
   T Sm = smin(vm - cm, u_hat - h.c_hat);
   T Sp = smax(vp + cp, u_hat + h.c_hat);
   if (T(0) <= Sm) {
-    phys_flux(eos, d, Vm, F);
+    phys_flux<PIN>(eos, d, Vm, F);
+    if (PIN & PIN_SUPERSONIC) split_normal(d, Vm, F);
   } else if (T(0) >= Sp) {
-    phys_flux(eos, d, Vp, F);
+    phys_flux<PIN>(eos, d, Vp, F);
+    if (PIN & PIN_SUPERSONIC) split_normal(d, Vp, F);
   } else {
     T Sstar = (Vp[4] - Vm[4] + Vm[0] * vm * (Sm - vm) - Vp[0] * vp * (Sp - vp)) /
               (Vm[0] * (Sm - vm) - Vp[0] * (Sp - vp));
     if (Sstar >= T(0))
-      hllc_fstar(eos, d, Vm, Sm, Sstar, F);
+      hllc_fstar<PIN>(eos, d, Vm, Sm, Sstar, F);
     else if (Sstar <= T(0))
-      hllc_fstar(eos, d, Vp, Sp, Sstar, F);
+      hllc_fstar<PIN>(eos, d, Vp, Sp, Sstar, F);
     else
       return ERR_HLLC;
   }
@@ -454,7 +620,7 @@ M2C_HD int flux_hllc(const Eos<T>& eos, int d, const T* Vm, const T* Vp, T* F) {
 // The dissipation sum runs over eigenvectors in the outer loop; for every
 // flux component the terms are still subtracted in eigenvector order 1..5,
 // as the reference's inner loop does.
-template <typename T>
+template <int PIN = 0, typename T>
 M2C_HD int flux_roe(const Eos<T>& eos, int d, const T* Vm, const T* Vp, T delta, T* F) {
   RoeHat<T> h;
   T sm0 = sqrt(Vm[0]), sp0 = sqrt(Vp[0]);
@@ -462,7 +628,7 @@ M2C_HD int flux_roe(const Eos<T>& eos, int d, const T* Vm, const T* Vp, T delta,
   vel[0] = roe_avg(sm0, Vm[1], sp0, Vp[1]);
   vel[1] = roe_avg(sm0, Vm[2], sp0, Vp[2]);
   vel[2] = roe_avg(sm0, Vm[3], sp0, Vp[3]);
-  T H = roe_avg(sm0, eos.enthalpy(Vm), sp0, eos.enthalpy(Vp));
+  T H = roe_avg(sm0, eos.template enthalpy<PIN | PIN_ENTHALPY>(Vm), sp0, eos.template enthalpy<PIN | PIN_ENTHALPY>(Vp));
   roe_hat(eos, d, Vm, Vp, h);
   const T c = h.c_hat, c2 = h.c_hat2, rho = h.rho_hat;
   const T drho = Vp[0] - Vm[0], dp = Vp[4] - Vm[4];
@@ -482,8 +648,8 @@ M2C_HD int flux_roe(const Eos<T>& eos, int d, const T* Vm, const T* Vp, T delta,
   for (int i = 0; i < 5; i++)
     if (fabs(lam[i]) < tol) lam[i] = (lam[i] * lam[i] + tol * tol) / (T(2) * tol);
   T fm[5];
-  phys_flux(eos, d, Vm, fm);
-  phys_flux(eos, d, Vp, F);
+  phys_flux<PIN | PIN_ENTHALPY>(eos, d, Vm, fm);
+  phys_flux<PIN | PIN_ENTHALPY>(eos, d, Vp, F);
   for (int i = 0; i < 5; i++) F[i] = T(0.5) * (fm[i] + F[i]);
   for (int p = 0; p < 5; p++) {
     // eigenvector p and its wave strength (FluxFcnBase.h:155-245, FluxFcnGenRoe.h:125-163)
@@ -520,20 +686,20 @@ M2C_HD int flux_roe(const Eos<T>& eos, int d, const T* Vm, const T* Vp, T delta,
 
 // Rusanov / LLF flux; also the material-interface variant with two EOS
 // (FluxFcnLLF.h:47-111, 119-185).
-template <typename T>
+template <int PIN = 0, typename T>
 M2C_HD int flux_llf2(const Eos<T>& em, const Eos<T>& ep, int d, const T* Vm, const T* Vp, T* F) {
   T e_m = em.energy(Vm[0], Vm[4]);
   T e_p = ep.energy(Vp[0], Vp[4]);
-  T c_m = em.c2(Vm[0], e_m);
+  T c_m = em.template c2<PIN>(Vm[0], e_m);
   if (c_m < T(0)) return ERR_SOUND;
   c_m = sqrt(c_m);
-  T c_p = ep.c2(Vp[0], e_p);
+  T c_p = ep.template c2<PIN>(Vp[0], e_p);
   if (c_p < T(0)) return ERR_SOUND;
   c_p = sqrt(c_p);
   T a = smax(fabs(vnorm(d, Vm)) + c_m, fabs(vnorm(d, Vp)) + c_p);
   T fm[5], fp[5], Um[5], Up[5];
-  phys_flux(em, d, Vm, fm);
-  phys_flux(ep, d, Vp, fp);
+  phys_flux<PIN>(em, d, Vm, fm);
+  phys_flux<PIN>(ep, d, Vp, fp);
   em.p2c(Vm, Um);
   ep.p2c(Vp, Up);
   for (int i = 0; i < 5; i++) F[i] = T(0.5) * ((fm[i] + fp[i]) - a * (Up[i] - Um[i]));

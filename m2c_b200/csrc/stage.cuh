@@ -17,32 +17,42 @@
 // they are rebuilt from interior cells by the boundary rule when loaded.
 //
 // Work decomposition: a CTA owns a 32 x TY column of cells and marches along
-// z through a chunk of planes, keeping a ring of 4 primitive planes (with a
-// 2-cell x/y halo) in shared memory. The stage's input is a primitive state
-// in the compute type (V^n for stage 1; for later stages clip(C2P(U_s)),
-// written by the previous stage's update), so planes are copied into the
-// ring as they lie in HBM and only ghost cells are rewritten by the boundary
-// rule. A plane of all five components lands with ONE tensor copy
-// (cp.async.bulk.tensor over a 4D map x, y, z, component of the
-// five-component buffer; box 40 x (TY+4) x 1 x 5 starting at x = i0-4, a
-// 16-byte boundary; completion counted on an mbarrier per ring slot),
-// issued by one thread; cells outside the domain in x/y arrive as zeros and
-// take their value from their image cell by the boundary rule. Where x or y
-// is periodic the halo wraps around the domain, which a tiled copy cannot
-// express; those launches copy each value with cp.async from its wrapped
-// position instead. Iteration m of the plane pipeline:
-//   (1) ghost rules on plane m+2 (landed), copy of plane m+3 into the
-//       slot plane m-1 has freed,
-//   (2) slopes + revert mask of every cell of plane m+1 (x -1..32, y -1..TY),
-//   (3) every face flux once: x/y faces of plane m and the z faces m+1/2,
-//   (4) residual + RK update of plane m (z faces m-1/2 and m+1/2 from the
-//       two-plane z-flux ring), writing the next stage's primitive input.
+// z through a chunk of planes, one warp per row of 32 cells. What the tile
+// needs beyond its own cells (the face states of the four halo sides, the
+// fluxes of its high x and y faces, the boundary rule on the halo, the plane
+// copies) is done by one more warp (StageShape::edge_warp), or spread over
+// the row warps as one extra item each.
+// The stage's input is a primitive state in the compute type (V^n for stage
+// 1; for later stages clip(C2P(U_s)), written by the previous stage's
+// update). Its planes lie in a shared-memory ring with a 2-cell x/y halo,
+// each brought in by ONE tensor copy of all five components
+// (cp.async.bulk.tensor over a 4D map x, y, z, component; box 40 x (TY+4) x
+// 1 x 5 starting at x = i0-4, a 16-byte boundary) on an mbarrier per slot
+// (and one more copy for the material IDs, box 64 x (TY+4) from x = i0-16).
+// Cells outside the domain in x/y arrive as zeros; one warp rewrites
+// them from their image or wrapped cell before any other warp reads them.
+// Ghost planes in z are not stored: a thread forms its column's ghost value.
+//
+// Iteration p of the plane pipeline:
+//   A(p)  slopes and checked face states of plane p, one direction after the
+//         other, into shared memory (the high z state stays in registers)
+//   barrier
+//   B(p)  the fluxes of plane p's low x and y faces (to shared memory) and of
+//         its low z face p-1/2; with it the update of plane p-1 is complete
+//   barrier
+//   C(p)  the sum of plane p's fluxes but the one of z face p+1/2, kept in
+//         registers for B(p+1)
+// The three directions and the three faces are loops that are not unrolled:
+// the kernel is bound by issue and by instruction fetch, and three copies of
+// the flux code cost more in fetch stalls than their selects save.
 // Face states follow Reconstructor.cpp: slope-limited primitive values, the
 // first face (in the order l,r,b,t,k,f) failing CheckState reverted to the
 // cell value, every face needing clipping reverted to the cell value, and a
 // remaining CheckState failure reported as an error (never a trap).
 #pragma once
 #include <cuda.h>  // CUtensorMap
+
+#include <type_traits>
 
 #include "physics.cuh"
 
@@ -54,6 +64,8 @@ constexpr int TX = 32;
 // columns i0-2 .. i0+33 plus two unused columns each side, so that the box
 // starts on a 16-byte boundary for 4- and 8-byte elements).
 constexpr int STAGE_TMA_BX = 40;
+// The same for the material-ID box: cells i0-16 .. i0+47 (one byte each).
+constexpr int STAGE_TMA_IX = 64;
 // Upper bound of mbarrier polls for one plane copy (a copy from valid
 // addresses always lands; the bound turns a fault into an error status).
 constexpr int STAGE_TMA_POLLS = 1 << 22;
@@ -84,8 +96,13 @@ struct Grid3 {
   // meshes), which then stand in for the arrays
   int lu[3];
   double lA0[3], lB0[3], lC0[3];
+  float fA0[3], fB0[3], fC0[3];  // the same in FP32
   int lK0[3];
 };
+
+template <typename T> __device__ __forceinline__ const T* axis_constant(const double* d, const float* f);
+template <> __device__ __forceinline__ const double* axis_constant<double>(const double* d, const float*) { return d; }
+template <> __device__ __forceinline__ const float* axis_constant<float>(const double*, const float* f) { return f; }
 
 struct SchemeK {
   int flux, limiter, rec_linear, slope_zero_at_interface;
@@ -169,8 +186,8 @@ struct StageArgs {
   IfaceView iface;
   ViscView visc;
   WallView wall;
-  int use_tma;           // planes by tensor copy (x and y not periodic, maps built)
   CUtensorMap tin;       // 4D map of the stage input (Pin as one five-component buffer)
+  CUtensorMap tid;       // 3D map of the material IDs
 };
 
 __device__ __forceinline__ void report(DevError* e, int code, int cell, int where) {
@@ -180,37 +197,28 @@ __device__ __forceinline__ void report(DevError* e, int code, int cell, int wher
   }
 }
 
-template <typename T, int TY>
-struct StageSmem {
-  static constexpr int RX = TX + 4, RY = TY + 4;   // loaded region: x -2..TX+1, y -2..TY+1
-  static constexpr int BX = STAGE_TMA_BX;          // stored columns: x -4..TX+3 (loaded column lx at lx + 2)
-  static constexpr int MX = TX + 2, MY = TY + 2;   // mask region: x -1..TX, y -1..TY
-  static constexpr int NFX = (TX + 1) * TY;        // x faces of a plane
-  static constexpr int NFY = TX * (TY + 1);        // y faces of a plane
-  static constexpr int NFZ = TX * TY;              // z faces between two planes
-  alignas(128) T v[4][5][RY][BX];  // ring of primitive planes, slot = plane & 3 (tensor-copy boxes)
-  T sig[2][3][5][MY][MX];     // limited slopes (x, y, z) of the mask region, two planes
-  T fx[5][NFX];
-  T fy[5][NFY];
-  T fz[2][5][NFZ];
-  uint8_t mask[2][MY][MX];
-  uint8_t real[4][RY][RX];    // 1 = real (interior or periodic image), 0 = ghost / unused
-  uint8_t ids[4][RY][RX];
-  double red[TY * TX / 32];
-  unsigned long long bar[4];  // one mbarrier per ring slot (tensor copies)
-};
+// Planes of the ring: three are read in an iteration (p-1, p, p+1) and one
+// is in flight.
+constexpr int STAGE_RING = 4;
 
-// Shared memory of one CTA. At a material interface face the left and the
-// right cell see different fluxes; only the left cell's is stored, and the
-// right cell's (NUMERICAL interface flux) is recomputed by that cell in the
-// update phase, so the two-material kernel needs no second set of flux tiles.
 template <typename T, int TY, bool MULTI>
-struct StageSmemAll {
-  StageSmem<T, TY> b;
+struct StageSmem {
+  static constexpr int RX = TX + 4, RY = TY + 4;  // loaded region: x -2..TX+1, y -2..TY+1
+  static constexpr int BX = STAGE_TMA_BX;         // cell (i0 + x, j0 + y) at column x + 4, row y + 2
+  // one plane each, on the 128-byte boundary that a tensor copy starts at
+  struct alignas(128) Plane { T v[5][RY][BX]; };
+  struct alignas(128) IdPlane { uint8_t v[RY][STAGE_TMA_IX]; };  // column x + 16
+  Plane v[STAGE_RING];
+  IdPlane id[MULTI ? STAGE_RING : 1];
+  // of the faces of a row or column of cells: hi the high-side state of the
+  // cell left of the face, lo the low-side state of the cell right of it, f
+  // the flux
+  T hix[5][TY][TX + 1], lox[5][TY][TX + 1], fx[5][TY][TX + 1];
+  T hiy[5][TY + 1][TX], loy[5][TY + 1][TX], fy[5][TY + 1][TX];
+  T loz[5][TY][TX];
+  double red[TY];
+  unsigned long long bar[STAGE_RING];  // one mbarrier per ring slot
 };
-
-// Value c of loaded cell (lx, ly) in ring slot sl.
-#define M2C_VV(sl, c, ly, lx) sm.v[sl][c][ly][(lx) + 2]
 
 // Resolve a possibly-outside index along one axis (at most two cells out).
 // Returns the interior index to read; sets ghost side (-1 none, 0 low, 1 high)
@@ -246,9 +254,13 @@ template <> struct EosPick<float> {
   __device__ static const Eos<float>& get(const SchemeK& s, int id) { return s.ef[id]; }
 };
 
-template <typename T, bool MULTI>
+// SG: every material is a stiffened gas (the kernel variant then carries no
+// other equation of state and no test of the kind).
+template <typename T, bool MULTI, bool SG = false>
 __device__ __forceinline__ const Eos<T>& eos_of(const SchemeK& s, int id) {
-  return EosPick<T>::get(s, MULTI ? (id < s.nmat ? id : 0) : 0);
+  const Eos<T>& e = EosPick<T>::get(s, MULTI ? (id < s.nmat ? id : 0) : 0);
+  if (SG) __builtin_assume(e.kind == EOS_SG);
+  return e;
 }
 
 // Boundary face state built from the interior neighbour's face state
@@ -277,59 +289,77 @@ __device__ __forceinline__ void ghost_face(int bc, int axis, const T* inner_face
   }
 }
 
-template <typename T, int FLUX>
+template <typename T, int FLUX, int PIN>
 __device__ __forceinline__ int flux_of(const Eos<T>& e, int d, const T* VL, const T* VR, T delta, T* F) {
-  if (FLUX == FLUX_HLLC) return flux_hllc(e, d, VL, VR, F);
-  if (FLUX == FLUX_ROE) return flux_roe(e, d, VL, VR, delta, F);
-  return flux_llf2(e, e, d, VL, VR, F);
+  if (FLUX == FLUX_HLLC) return flux_hllc<PIN>(e, d, VL, VR, F);
+  if (FLUX == FLUX_ROE) return flux_roe<PIN>(e, d, VL, VR, delta, F);
+  return flux_llf2<PIN>(e, e, d, VL, VR, F);
 }
 
-// Asynchronous 8-byte global -> shared copy (cp.async, L1-allocating) and
-// its completion wait; used to prefetch the next plane while the current one
-// is being computed.
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
+// Primitive state of a ghost cell beyond a boundary of type bc on `axis`
+// from its image cell's (SpaceOperator::ApplyBoundaryConditions).
 template <typename T>
-__device__ __forceinline__ void cp_async_t(T* smem, const T* gmem) {
-  if constexpr (sizeof(T) == 8) cp_async8(smem, gmem);
-  else cp_async4(smem, gmem);
+__device__ __forceinline__ void ghost_cell(const Grid3& g, int axis, int bc, const T* image, T* out) {
+#pragma unroll
+  for (int c = 0; c < 5; c++) out[c] = image[c];
+  if (bc == BC_INLET) {
+#pragma unroll
+    for (int c = 0; c < 5; c++) out[c] = T(g.inlet[c]);
+  } else if (bc == BC_OUTLET) {
+#pragma unroll
+    for (int c = 0; c < 5; c++) out[c] = T(g.outlet[c]);
+  } else if (bc == BC_STICKWALL) {
+    out[1] = -out[1]; out[2] = -out[2]; out[3] = -out[3];
+  } else {  // SYMMETRY / SLIPWALL: normal velocity flipped
+    if (axis == 0) out[1] = -out[1];
+    else if (axis == 1) out[2] = -out[2];
+    else out[3] = -out[3];
+  }
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Resident CTAs per SM each instantiation is compiled for. The FP32 kernel
-// runs 32 x 16 tiles, one 512-thread CTA per SM (126 registers); measured
-// against 32 x 8 tiles at two CTAs per SM it is 2.5% faster on the 256^3 box
-// (less halo work, same 16 warps), and 32 x 4 tiles at four CTAs per SM are
-// 25% slower.
-template <typename T> struct StageOcc { static constexpr int value = 1; };
-#ifndef M2C_STAGE_OCC_F32
-#define M2C_STAGE_OCC_F32 1
-#endif
-template <> struct StageOcc<float> { static constexpr int value = M2C_STAGE_OCC_F32; };
+// Tile rows, whether an extra warp does the edge work, and the CTAs per SM
+// that the kernel is compiled for. Registers are handed out per quarter of an
+// SM, so warps per SM come in fours: 12 (11 rows and the edge warp) leave 168
+// registers each, which the FP64 kernel needs to run without spills; 16 leave
+// 128, which the FP32 kernel fits as two CTAs of 8 rows. Measured per stage
+// launch, before -> now (the kernel before: 32 x 8 tiles in FP64 and 32 x 16
+// in FP32 at one CTA per SM, all slopes kept in shared memory, short-cut
+// tests and a branch per limiter component): FP64 HLLC channel 161x97x131
+// 1.76 -> 0.92 ms, FP64 bubble 101x96x90 1.50 -> 0.64 ms, mixed bubble cluster
+// 192^3 1.91 -> 1.41 ms, mixed HLLC box 160^3 0.78 -> 0.60 ms, mixed Roe box
+// 256^3 2.47 -> 2.29 ms. FP64 with 8 rows and the edge warp is 1.39 ms on the
+// channel, with 7 rows (255 registers) 1.45 ms; FP32 with 16 rows at one CTA
+// per SM 8 % slower on the 256^3 box.
+template <typename T> struct StageShape {
+  static constexpr int ty = 11, warps = ty + 1, occ = 1;
+  static constexpr bool edge_warp = true;
+};
+template <> struct StageShape<float> {
+  static constexpr int ty = 8, warps = ty, occ = 2;
+  static constexpr bool edge_warp = false;
+};
 
 // CONS: reconstruction in conservative or characteristic variables (a
 // separate instantiation so the primitive-variable kernels carry none of it).
 // WALLS (two-material variant only): the branch of faces cut by an embedded
 // surface is compiled in; without it the kernel carries none of its tests.
-template <typename T, int TY, int FLUX, bool MULTI, bool CONS, bool WALLS = false>
-__global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(const __grid_constant__ StageArgs a) {
+template <typename T, int FLUX, bool MULTI, bool CONS, bool WALLS, bool SG>
+__global__ void __launch_bounds__(TX * StageShape<T>::warps, CONS ? 1 : StageShape<T>::occ)
+    stage_kernel(const __grid_constant__ StageArgs a) {
+  constexpr int TY = StageShape<T>::ty;
+  constexpr bool EW = StageShape<T>::edge_warp;
+  constexpr int PIN = PIN_MOMENTUM | PIN_SOUND | (MULTI ? PIN_SUPERSONIC : 0);  // FP32, see physics.cuh
+  static_assert(TY >= 6 && TY <= 16, "one warp holds both x-halo columns of the tile; the spread extra items take warps 0 to 5");
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  typedef StageSmem<T, TY> S;
-  typedef StageSmemAll<T, TY, MULTI> SA;
-  SA& all = *reinterpret_cast<SA*>(smem_raw);
-  S& sm = all.b;
+  typedef StageSmem<T, TY, MULTI> S;
+  S& sm = *reinterpret_cast<S*>(smem_raw);
+  constexpr int RING = STAGE_RING;
+  constexpr int CS = S::RY * S::BX;  // component stride of a plane
+  constexpr int XS = TY * (TX + 1), YS = (TY + 1) * TX, ZS = TY * TX;  // and of the x, y and z face arrays
   const Grid3& g = a.g;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  constexpr int NT = TX * TY;
-  constexpr int NLOAD = S::RY * S::RX;
-  constexpr int LPT = (NLOAD + NT - 1) / NT;  // loaded cells per thread
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const bool edge = EW && row == TY;                // the edge warp
+  const bool copier = lane == 0 && row == (EW ? TY : 5);  // the thread that starts the plane copies
   const bool xper = g.bc[0] == BC_PERIODIC, yper = g.bc[2] == BC_PERIODIC, zper = g.bc[4] == BC_PERIODIC;
   const double dt = a.clock[1];
   const double bdt = a.bdt_coef * dt;
@@ -339,105 +369,49 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
   const int limiter = a.s.limiter;
   const bool rec_linear = a.s.rec_linear;
   const bool slope_zero = MULTI && a.s.slope_zero_at_interface;
+  const bool face_pass = MULTI && (a.iface.faces_out || (WALLS && a.wall.faces_out));
 
-  int i0 = 0, j0 = 0;  // tile origin of the current work item
-  uint8_t idreg[LPT];
-  // Plane copies: tensor copies unless x or y is periodic (CTA-uniform).
-  const bool use_tma = a.use_tma != 0;
-  constexpr unsigned TMA_BYTES = 5u * S::RY * S::BX * sizeof(T);
+  int i0 = 0, j0 = 0, pbase = 0;  // tile origin and first plane of the current segment
+  constexpr unsigned TMA_BYTES = 5u * S::RY * S::BX * sizeof(T) + (MULTI ? unsigned(S::RY) * STAGE_TMA_IX : 0u);
   unsigned tma_phase = 0;  // bit s: parity of the next completion of slot s's mbarrier
-  if (use_tma) {
-    if (tid == 0) {
-      for (int q = 0; q < 4; q++) {
-        const unsigned bar = (unsigned)__cvta_generic_to_shared(&sm.bar[q]);
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-      }
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(&a.tin)) : "memory");
+  if (copier) {
+    for (int q = 0; q < RING; q++) {
+      const unsigned bar = (unsigned)__cvta_generic_to_shared(&sm.bar[q]);
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
     }
-    __syncthreads();
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(&a.tin)) : "memory");
   }
 
-  auto slot4 = [](int p) { return p & 3; };
-  auto plane_is_ghost = [&](int p) { return !zper && (p < 0 || p >= g.nz); };
+  auto slot_of = [&](int p) { return int(unsigned(p - pbase) % unsigned(RING)); };
+  auto real_plane = [&](int p) { return zper || (p >= 0 && p < g.nz); };
 
-  // Per tile, for each loaded cell of this thread: its in-plane offset (the
-  // image cell for ghosts, the wrapped cell for periodic halos) and its kind
-  // in x and y: bits 0-1 x ghost side + 1 (0 none, 1 low, 2 high), bits 2-3
-  // the same for y, bit 4 far (outside by more than one cell, not periodic).
-  int xyoff[LPT];
-  uint8_t xyinfo[LPT];
-  auto tile_setup = [&]() {
-#pragma unroll
-    for (int r = 0; r < LPT; r++) {
-      const int q = tid + r * NT;
-      if (q >= NLOAD) break;
-      const int ly = q / S::RX, lx = q - ly * S::RX;
-      int sx, sy;
-      bool far = false;
-      const int ii = resolve_axis(i0 + lx - 2, g.nx, xper, sx, far);
-      const int jj = resolve_axis(j0 + ly - 2, g.ny, yper, sy, far);
-      xyoff[r] = jj * (int)g.px + ii;
-      xyinfo[r] = uint8_t((sx + 1) | ((sy + 1) << 2) | (far ? 16 : 0));
-    }
-  };
-
-  // (1a) start copying plane p into its ring slot. Tensor path: one thread
-  // issues the plane's copy (all components) against the slot's mbarrier,
-  // after a proxy fence orders the slot's earlier generic accesses (every
-  // thread passed a barrier since) before the asynchronous write. Element
-  // path (periodic x or y): one cp.async per value from the image or
-  // wrapped position.
+  // Start copying plane p into its ring slot (one thread,
+  // after a barrier that ends every read of the slot's previous plane).
   auto issue_plane = [&](int p) {
-    int sz;
-    bool farz = false;
-    const int kk = resolve_axis(p, g.nz, zper, sz, farz);
-    const int s = slot4(p);
-    if (use_tma) {
-      if (tid == 0) {
-        const unsigned bar = (unsigned)__cvta_generic_to_shared(&sm.bar[s]);
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(&sm.v[s][0][0][0]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(TMA_BYTES) : "memory");
-        asm volatile(
-            "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-            "[%6];" ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(&a.tin)), "r"(i0 - 4), "r"(j0 - 2), "r"(kk),
-            "r"(0), "r"(bar)
-            : "memory");
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < LPT; r++) {
-        const int q = tid + r * NT;
-        if (q >= NLOAD) break;
-        const int ly = q / S::RX, lx = q - ly * S::RX;
-        const long long off = (long long)kk * g.plane + xyoff[r];
-#pragma unroll
-        for (int c = 0; c < 5; c++) cp_async_t(&M2C_VV(s, c, ly, lx), static_cast<const T*>(a.Pin[c]) + off);
-      }
-      cp_async_commit();
-    }
-    if (MULTI) {
-#pragma unroll
-      for (int r = 0; r < LPT; r++) {
-        const int q = tid + r * NT;
-        if (q >= NLOAD) break;
-        idreg[r] = a.id[(long long)kk * g.plane + xyoff[r]];
-      }
+    const int s = slot_of(p), kk = zper ? wrap_index(p, g.nz) : p;
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(&sm.bar[s]);
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(&sm.v[s].v[0][0][0]);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(TMA_BYTES) : "memory");
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(&a.tin)), "r"(i0 - 4), "r"(j0 - 2), "r"(kk),
+        "r"(0), "r"(bar)
+        : "memory");
+    if constexpr (MULTI) {
+      const unsigned idst = (unsigned)__cvta_generic_to_shared(&sm.id[s].v[0][0]);
+      asm volatile(
+          "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+          "[%5];" ::"r"(idst), "l"(reinterpret_cast<unsigned long long>(&a.tid)), "r"(i0 - 16), "r"(j0 - 2), "r"(kk),
+          "r"(bar)
+          : "memory");
     }
   };
 
-  // (1b) wait for plane p, then a CTA barrier (which also keeps the plane's
-  // commit from overwriting ids and kinds the previous iteration's update
-  // still reads). Tensor path: every thread polls the slot's mbarrier
-  // (bounded; a copy that never lands is reported and the CTA stops).
+  // Wait for plane p (bounded; a copy that never lands is reported and the
+  // CTA stops at the next barrier). Every thread waits for every plane once.
   auto wait_plane = [&](int p) -> bool {
-    if (!use_tma) {
-      cp_async_wait_all();
-      __syncthreads();
-      return true;
-    }
-    const int s = slot4(p);
+    const int s = slot_of(p);
     const unsigned bar = (unsigned)__cvta_generic_to_shared(&sm.bar[s]);
     const unsigned parity = (tma_phase >> s) & 1u;
     unsigned ok = 0;
@@ -450,74 +424,65 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
     }
     tma_phase ^= 1u << s;
     if (!ok) report(a.err, ERR_ITER_CAP, -1, where + 5);
-    __syncthreads();
     return ok != 0;
   };
 
-  // (1c) the landed plane: boundary rule on ghost cells
-  // (SpaceOperator::ApplyBoundaryConditions), cell kinds and ids. A ghost
-  // cell takes its image cell's value (the element path copied it there; the
-  // tensor path reads it from the neighbour in x or y, or finds it in place
-  // for a ghost plane in z), then the rule of its face.
-  auto commit_plane = [&](int p) {
-    const int s = slot4(p);
-    int sz;
-    bool farz = false;
-    resolve_axis(p, g.nz, zper, sz, farz);
-#pragma unroll
-    for (int r = 0; r < LPT; r++) {
-      const int q = tid + r * NT;
-      if (q >= NLOAD) break;
-      const int ly = q / S::RX, lx = q - ly * S::RX;
-      const int gx = xyinfo[r] & 3, gy = (xyinfo[r] >> 2) & 3;
-      const bool far = (xyinfo[r] & 16) || farz;
-      const int nghost = (gx != 0) + (gy != 0) + (sz >= 0);
-      const bool real = nghost == 0 && !far;
-      if (nghost == 1 && !far) {
-        const int axis = gx ? 0 : (gy ? 1 : 2);
-        const int side = gx ? gx - 1 : (gy ? gy - 1 : sz);
-        const int bc = g.bc[2 * axis + side];
-        if (use_tma && axis < 2 && bc != BC_INLET && bc != BC_OUTLET) {
-          const int ix = axis == 0 ? lx + (side ? -1 : 1) : lx, iy = axis == 1 ? ly + (side ? -1 : 1) : ly;
-#pragma unroll
-          for (int c = 0; c < 5; c++) M2C_VV(s, c, ly, lx) = M2C_VV(s, c, iy, ix);
-        }
-        if (bc == BC_INLET) {
-#pragma unroll
-          for (int c = 0; c < 5; c++) M2C_VV(s, c, ly, lx) = T(g.inlet[c]);
-        } else if (bc == BC_OUTLET) {
-#pragma unroll
-          for (int c = 0; c < 5; c++) M2C_VV(s, c, ly, lx) = T(g.outlet[c]);
-        } else if (bc == BC_STICKWALL) {
-          M2C_VV(s, 1, ly, lx) = -M2C_VV(s, 1, ly, lx);
-          M2C_VV(s, 2, ly, lx) = -M2C_VV(s, 2, ly, lx);
-          M2C_VV(s, 3, ly, lx) = -M2C_VV(s, 3, ly, lx);
-        } else {  // SYMMETRY / SLIPWALL: normal velocity flipped
-          M2C_VV(s, 1 + axis, ly, lx) = -M2C_VV(s, 1 + axis, ly, lx);
-        }
+  // The landed plane p (a real one): the loaded cells outside the domain in
+  // x or y, shared by all threads. A cell beyond a periodic boundary takes its wrapped
+  // cell's value, one beyond another boundary the value the boundary rule
+  // gives it from its image cell; both are read from global memory. Cells
+  // outside twice, or by more than one cell, are never read.
+  int fcl = 0, frl = 0, fncol = 0, fn = 0;  // columns and rows below 0, cells of the outside columns, of all (per tile)
+  auto fix_plane = [&](int p) {
+    const int s = slot_of(p), kk = zper ? wrap_index(p, g.nz) : p;
+    for (int it = row * TX + lane; it < fn; it += TX * StageShape<T>::warps) {
+      int x, y;  // cell relative to the tile's origin
+      if (it < fncol) {
+        const int q = it / S::RY;
+        x = q < fcl ? q - 2 : g.nx - i0 + q - fcl;
+        y = it - q * S::RY - 2;
+      } else {
+        const int q = (it - fncol) / S::RX;
+        y = q < frl ? q - 2 : g.ny - j0 + q - frl;
+        x = (it - fncol) - q * S::RX - 2;
       }
-      sm.real[s][ly][lx] = real ? 1 : 0;
-      sm.ids[s][ly][lx] = MULTI ? idreg[r] : 0;
+      int sx, sy;
+      bool far = false;
+      const int ii = resolve_axis(i0 + x, g.nx, xper, sx, far), jj = resolve_axis(j0 + y, g.ny, yper, sy, far);
+      if (far || (sx >= 0 && sy >= 0)) continue;
+      const long long off = (long long)kk * g.plane + (long long)jj * g.px + ii;
+      T v[5], o[5];
+#pragma unroll
+      for (int c = 0; c < 5; c++) v[c] = static_cast<const T*>(a.Pin[c])[off];
+      if (MULTI) sm.id[s].v[y + 2][x + 16] = a.id[off];
+      const int axis = sx >= 0 ? 0 : 1, side = sx >= 0 ? sx : sy;
+      if (side >= 0) {
+        ghost_cell(g, axis, g.bc[2 * axis + side], v, o);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 5; c++) o[c] = v[c];
+      }
+#pragma unroll
+      for (int c = 0; c < 5; c++) sm.v[s].v[c][y + 2][x + 4] = o[c];
     }
-    // order this thread's generic writes to the slot before the tensor copy
-    // that refills it four planes later
-    if (use_tma) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // order these writes before the tensor copy that refills the slot
+    if (fn) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   };
 
-  // Limiter coefficients (Reconstructor::Setup) of the cell at loaded
-  // position (lx, ly) of plane p along axis d: the axis' constants on a
-  // uniform axis, else its per-index arrays. The generalized minmod uses
-  // C = B/(A+1) only (carried in B).
-  auto limiter_coeffs = [&](int p, int lx, int ly, int d, T& A, T& B, int& K) {
+  // Limiter coefficients (Reconstructor::Setup) of the cell at column cx,
+  // row cy of plane p along axis d: the axis' constants on a uniform axis,
+  // else its per-index arrays. The generalized minmod uses C = B/(A+1) only
+  // (carried in B).
+  auto limiter_coeffs = [&](int p, int cx, int cy, int d, T& A, T& B, int& K) {
     if (g.lu[d]) {
       if (limiter == LIM_VANALBADA) {
-        A = T(g.lA0[d]); B = T(g.lB0[d]); K = g.lK0[d];
+        A = axis_constant<T>(g.lA0, g.fA0)[d]; B = axis_constant<T>(g.lB0, g.fB0)[d]; K = g.lK0[d];
       } else {
-        A = T(0); B = T(g.lC0[d]);
+        A = T(0); B = axis_constant<T>(g.lC0, g.fC0)[d];
       }
       return;
     }
-    const int ix = d == 0 ? wrap_index(i0 + lx - 2, g.nx) : (d == 1 ? wrap_index(j0 + ly - 2, g.ny)
+    const int ix = d == 0 ? wrap_index(i0 + cx - 4, g.nx) : (d == 1 ? wrap_index(j0 + cy - 2, g.ny)
                                                                     : wrap_index(p, g.nz));
     if (limiter == LIM_VANALBADA) {
       A = T(g.lA[d][ix]); B = T(g.lB[d][ix]); K = g.lK[d][ix];
@@ -526,76 +491,120 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
     }
   };
 
-  // Limited slopes in direction d of the real cell at loaded position
-  // (lx, ly) of plane p (needs planes p-1, p, p+1 for d = 2).
-  auto slopes = [&](int p, int lx, int ly, int d, T* sd) {
-    const int s0 = slot4(p);
-    int sm1 = s0, sp1 = s0, lxm = lx, lxp = lx, lym = ly, lyp = ly;
-    if (d == 0) { lxm = lx - 1; lxp = lx + 1; }
-    else if (d == 1) { lym = ly - 1; lyp = ly + 1; }
-    else { sm1 = slot4(p - 1); sp1 = slot4(p + 1); }
+  // States (and IDs) of the two neighbours along d of the cell at (cx, cy)
+  // of plane p, whose own state is v; ghost planes by the boundary rule.
+  auto neighbours = [&](int d, int p, int cx, int cy, const T* v, T* vm, T* vp, int& idm, int& idp) {
+    const int s0 = slot_of(p);
+    int sm1 = s0, sp1 = s0;
+    bool rm = true, rp = true;
+    if (d == 2) {
+      rm = real_plane(p - 1);
+      rp = real_plane(p + 1);
+      if (rm) sm1 = slot_of(p - 1);
+      if (rp) sp1 = slot_of(p + 1);
+    }
+    const int off = cy * S::BX + cx, step = d == 0 ? 1 : (d == 1 ? S::BX : 0);
+    const T* qm = &sm.v[sm1].v[0][0][0] + (off - step);
+    const T* qp = &sm.v[sp1].v[0][0][0] + (off + step);
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      vm[c] = qm[c * CS];
+      vp[c] = qp[c * CS];
+    }
+    if (!rm) ghost_cell(g, 2, g.bc[4], v, vm);
+    if (!rp) ghost_cell(g, 2, g.bc[5], v, vp);
+    if (MULTI && (WALLS || CONS || slope_zero)) {
+      const int ox = d == 0 ? 1 : 0, oy = d == 1 ? 1 : 0;
+      idm = sm.id[sm1].v[cy - oy][cx - ox + 12];
+      idp = sm.id[sp1].v[cy + oy][cx + ox + 12];
+    }
+  };
+
+  // Limited slopes in direction d of the real cell at (cx, cy) of plane p.
+  auto slopes = [&](int d, int p, int cx, int cy, int id, const T* v, T* sd) {
     if (!rec_linear) {
 #pragma unroll
       for (int c = 0; c < 5; c++) sd[c] = T(0);
       return;
     }
+    T vm[5], vp[5];
+    int idm = 0, idp = 0;
+    neighbours(d, p, cx, cy, v, vm, vp, idm, idp);
     T A, B;
     int K = 0;
-    limiter_coeffs(p, lx, ly, d, A, B, K);
-    bool zero = false;
-    if (slope_zero) {
-      const uint8_t id = sm.ids[s0][ly][lx];
-      zero = id != sm.ids[sm1][lym][lxm] || id != sm.ids[sp1][lyp][lxp];
-    }
+    limiter_coeffs(p, cx, cy, d, A, B, K);
+    const bool zero = slope_zero && (id != idm || id != idp);
     // no difference toward an inactive neighbour (Reconstructor.cpp:475-502)
-    const bool offm = WALLS && sm.ids[sm1][lym][lxm] == a.s.nmat;
-    const bool offp = WALLS && sm.ids[sp1][lyp][lxp] == a.s.nmat;
+    const bool offm = WALLS && idm == a.s.nmat, offp = WALLS && idp == a.s.nmat;
+    T dm[5], dp[5];
 #pragma unroll
     for (int c = 0; c < 5; c++) {
-      const T vc = M2C_VV(s0, c, ly, lx);
-      const T dm = offm ? T(0) : vc - M2C_VV(sm1, c, lym, lxm);
-      const T dp = offp ? T(0) : M2C_VV(sp1, c, lyp, lxp) - vc;
-      T sl = limited_slope_c(limiter, A, B, K, alpha, dm, dp);
-      sd[c] = zero ? T(0) : sl;
+      dm[c] = offm ? T(0) : v[c] - vm[c];
+      dp[c] = offp ? T(0) : vp[c] - v[c];
+    }
+    limited_slopes(limiter, A, B, K, alpha, dm, dp, sd);
+    if (slope_zero && zero) {
+#pragma unroll
+      for (int c = 0; c < 5; c++) sd[c] = T(0);
     }
   };
 
-  // Limited slopes in direction d of the real cell at (lx, ly) of plane p in
+  // Face states of the real cell at (cx, cy) of plane p along d: lo = v - s/2
+  // on its low face, hi = v + s/2 on its high one, each reverted to the cell
+  // value v where the reference reverts it. chain carries "a non-physical
+  // face was reverted already" from one direction of the cell to the next
+  // (faces in the reference's order l, r, b, t, k, f).
+  auto face_states = [&](int d, int p, int cx, int cy, int id, const Eos<T>& e, const T* v, bool& chain, int& err,
+                         T* lo, T* hi) {
+    T sd[5];
+    slopes(d, p, cx, cy, id, v, sd);
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      lo[c] = v[c] - T(0.5) * sd[c];
+      hi[c] = v[c] + T(0.5) * sd[c];
+    }
+    if (e.both_fine(v, sd)) return;
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+      T* f = side ? hi : lo;
+      const bool bad = e.bad(f);
+      bool reverted = false;
+      // Reconstructor.cpp:719-775: only the first non-physical face is reverted.
+      if (!chain && bad) { reverted = true; chain = true; }
+      // SpaceOperator.cpp:3240-3273: a face needing clipping reverts to the cell value.
+      if (!reverted && e.needs_clip(f)) reverted = true;
+      // SpaceOperator.cpp:3275-3277: a face still non-physical is fatal.
+      if (!reverted && bad) err = ERR_STATE;
+      if (reverted) {
+#pragma unroll
+        for (int c = 0; c < 5; c++) f[c] = v[c];
+      }
+    }
+  };
+
+  // Limited slopes in direction d of the real cell at (cx, cy) of plane p in
   // the scheme's non-primitive variables (Reconstructor.cpp:397-404, 469-651):
   // differences of the conservative variables (rv 1, 3; neighbours converted
   // with their own EOS) or of the primitive ones (rv 2), projected on the
   // characteristic basis at the cell state (rv 2, 3) and limited there, then
   // mapped back. u is the cell's conservative state. Returns false where the
   // basis does not exist (c^2 < 0; the reference aborts).
-  auto nonprim_slopes = [&](int p, int lx, int ly, int d, int rv, const Eos<T>& e, const T* v, const T* u,
+  auto nonprim_slopes = [&](int d, int p, int cx, int cy, int id, int rv, const Eos<T>& e, const T* v, const T* u,
                             T* sd) -> bool {
-    const int s0 = slot4(p);
-    int sm1 = s0, sp1 = s0, lxm = lx, lxp = lx, lym = ly, lyp = ly;
-    if (d == 0) { lxm = lx - 1; lxp = lx + 1; }
-    else if (d == 1) { lym = ly - 1; lyp = ly + 1; }
-    else { sm1 = slot4(p - 1); sp1 = slot4(p + 1); }
     T A, B;
     int K = 0;
-    limiter_coeffs(p, lx, ly, d, A, B, K);
-    const uint8_t idm = sm.ids[sm1][lym][lxm], idp = sm.ids[sp1][lyp][lxp];
-    bool zero = false;
-    if (slope_zero) {
-      const uint8_t id = sm.ids[s0][ly][lx];
-      zero = id != idm || id != idp;
-    }
+    limiter_coeffs(p, cx, cy, d, A, B, K);
     T qm[5], qp[5], dl[5], dr[5];
-#pragma unroll
-    for (int c = 0; c < 5; c++) {
-      qm[c] = M2C_VV(sm1, c, lym, lxm);
-      qp[c] = M2C_VV(sp1, c, lyp, lxp);
-    }
+    int idm = 0, idp = 0;
+    neighbours(d, p, cx, cy, v, qm, qp, idm, idp);
+    const bool zero = slope_zero && (id != idm || id != idp);
     const bool uspace = rv != 2;
     if (uspace) {
       T t[5];
-      eos_of<T, MULTI>(a.s, idm).p2c(qm, t);
+      eos_of<T, MULTI, SG>(a.s, idm).p2c(qm, t);
 #pragma unroll
       for (int c = 0; c < 5; c++) qm[c] = t[c];
-      eos_of<T, MULTI>(a.s, idp).p2c(qp, t);
+      eos_of<T, MULTI, SG>(a.s, idp).p2c(qp, t);
 #pragma unroll
       for (int c = 0; c < 5; c++) qp[c] = t[c];
     }
@@ -634,54 +643,20 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
     return ok;
   };
 
-  // (2) slopes and revert bits of the real cell at mask-region (mx, my) of
-  // plane p. A cell of the tile (own) gets all three directions; a halo cell
-  // only the direction dh (0: x, 1: y) across which the tile's faces read it
-  // (x-halo cells feed only the tile's x faces, y-halo cells its y faces).
-  // Its revert bits then follow the revert rule below for that direction's
-  // two faces alone; the rule differs from the full cell's only where two
-  // faces are non-physical, which the cell's own tile reports as an error.
-  // Revert bits: bit 2d + side (0 minus face, 1 plus face), 0x40 for a
-  // conservative-variable face state.
-  auto mask_cell = [&](int p, int mx, int my, bool own, int dh) {
-    const int s0 = slot4(p), ms = p & 1;
-    const int ly = my + 1, lx = mx + 1;  // position in the loaded region
-    if (!sm.real[s0][ly][lx]) {
-      sm.mask[ms][my][mx] = 0;
-      return;
-    }
-    const uint8_t id = sm.ids[s0][ly][lx];
-    if (WALLS && id == a.s.nmat) {
-      // inactive: constant reconstruction, no checks (Reconstructor.cpp:452-462,
-      // SpaceOperator.cpp:3236-3237)
-      for (int d = 0; d < 3; d++)
-#pragma unroll
-        for (int c = 0; c < 5; c++) sm.sig[ms][d][c][my][mx] = T(0);
-      sm.mask[ms][my][mx] = 0;
-      return;
-    }
-    const Eos<T>& e = eos_of<T, MULTI>(a.s, id);
-    T v[5];
-#pragma unroll
-    for (int c = 0; c < 5; c++) v[c] = M2C_VV(s0, c, ly, lx);
-    uint8_t m = 0;
-    int err = ERR_NONE;
-    bool cons = false;
-    if (CONS && rec_linear) {
-      // non-primitive variables; any non-physical face sends the cell back
-      // to primitive variables (the RETRY of Reconstructor.cpp:719-775).
-      // Halo cells take this path whole (the tile's cells and its halo ring).
-      T sx[5], sy[5], sz[5];
+  // CONS: the two face states along dir of the real cell at (cx, cy) of plane
+  // p. Any non-physical face of the six sends the cell back to primitive
+  // variables (the RETRY of Reconstructor.cpp:719-775), so all are formed.
+  auto cons_states = [&](int dir, int p, int cx, int cy, int id, const Eos<T>& e, const T* v, int& err, T* lo, T* hi) {
+    if (rec_linear) {
+      T sx[5], sy[5], sz[5], u[5];
       const int rv = a.s.rec_var;
       const bool uspace = rv != 2;
-      T u[5];
       e.p2c(v, u);
-      bool okb = nonprim_slopes(p, lx, ly, 0, rv, e, v, u, sx);
-      okb = nonprim_slopes(p, lx, ly, 1, rv, e, v, u, sy) && okb;
-      okb = nonprim_slopes(p, lx, ly, 2, rv, e, v, u, sz) && okb;
+      bool okb = nonprim_slopes(0, p, cx, cy, id, rv, e, v, u, sx);
+      okb = nonprim_slopes(1, p, cx, cy, id, rv, e, v, u, sy) && okb;
+      okb = nonprim_slopes(2, p, cx, cy, id, rv, e, v, u, sz) && okb;
       if (!okb) err = ERR_SOUND;
-      cons = true;
-      uint8_t clipm = 0;
+      bool cons = true;
 #pragma unroll
       for (int q = 0; q < 6; q++) {
         const T* sg = q < 2 ? sx : (q < 4 ? sy : sz);
@@ -695,142 +670,67 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
 #pragma unroll
           for (int c = 0; c < 5; c++) f[c] = (q & 1) ? v[c] + T(0.5) * sg[c] : v[c] - T(0.5) * sg[c];
         }
-        if (e.bad(f)) cons = false;
-        else if (e.needs_clip(f)) clipm |= uint8_t(1u << q);  // SpaceOperator.cpp:3240-3273
-      }
-      if (cons) {
-        m = uint8_t(clipm | (uspace ? 0x40 : 0));
+        const bool bad = e.bad(f);
+        if (bad) cons = false;
+        if ((q >> 1) != dir) continue;
+        const bool rev = !bad && e.needs_clip(f);  // SpaceOperator.cpp:3240-3273
+        T* out = (q & 1) ? hi : lo;
 #pragma unroll
-        for (int c = 0; c < 5; c++) {
-          sm.sig[ms][0][c][my][mx] = sx[c];
-          sm.sig[ms][1][c][my][mx] = sy[c];
-          sm.sig[ms][2][c][my][mx] = sz[c];
-        }
+        for (int c = 0; c < 5; c++) out[c] = rev ? v[c] : f[c];
       }
+      if (cons) return;
     }
-    if (!cons) {
-      // primitive slopes direction by direction, each direction's faces in
-      // the reference's order (l, r, b, t, k, f)
-      const int dlo = (own || CONS) ? 0 : dh, dhi = (own || CONS) ? 2 : dh;
-      bool chain_done = false;
+    bool chain = false;
 #pragma unroll 1
-      for (int d = dlo; d <= dhi; d++) {
-        T sd[5];
-        slopes(p, lx, ly, d, sd);
-#pragma unroll
-        for (int c = 0; c < 5; c++) sm.sig[ms][d][c][my][mx] = sd[c];
-#pragma unroll
-        for (int side = 0; side < 2; side++) {
-          T f[5];
-#pragma unroll
-          for (int c = 0; c < 5; c++) f[c] = side ? v[c] + T(0.5) * sd[c] : v[c] - T(0.5) * sd[c];
-          const bool bad = e.bad(f);
-          bool reverted = false;
-          // Reconstructor.cpp:719-775: only the first non-physical face is reverted.
-          if (!chain_done && bad) { reverted = true; chain_done = true; }
-          // SpaceOperator.cpp:3240-3273: a face needing clipping reverts to the cell value.
-          if (!reverted && e.needs_clip(f)) reverted = true;
-          if (reverted) m |= uint8_t(1u << (2 * d + side));
-          // SpaceOperator.cpp:3275-3277: a face still non-physical is fatal.
-          else if (bad) err = ERR_STATE;
-        }
-      }
-    }
-    sm.mask[ms][my][mx] = m;
-    if (err && (own || CONS)) {
-      const int ka = wrap_index(p, g.nz);
-      const int ia = wrap_index(i0 + mx - 1, g.nx), ja = wrap_index(j0 + my - 1, g.ny);
-      report(a.err, err, (int)(((long long)ka * g.ny + ja) * g.nx + ia), where + 1);
-    }
-  };
-
-  // Final face state of the real cell at mask-region (mx,my) of plane p:
-  // direction d, side 0 = minus face (v - s/2), 1 = plus face (v + s/2).
-  auto cell_face = [&](int p, int mx, int my, int d, int side, T* out) {
-    const int s0 = slot4(p), ms = p & 1;
-    const uint8_t mk = sm.mask[ms][my][mx];
-    const bool rev = (mk >> (2 * d + side)) & 1u;
-    if (CONS && (mk & 0x40)) {  // conservative-variable face state
-      T v[5], u[5], uf[5];
-#pragma unroll
-      for (int c = 0; c < 5; c++) v[c] = M2C_VV(s0, c, my + 1, mx + 1);
-      if (rev) {
-#pragma unroll
-        for (int c = 0; c < 5; c++) out[c] = v[c];
-        return;
-      }
-      const Eos<T>& e = eos_of<T, MULTI>(a.s, sm.ids[s0][my + 1][mx + 1]);
-      e.p2c(v, u);
+    for (int d = 0; d < 3; d++) {
+      T l[5], h[5];
+      face_states(d, p, cx, cy, id, e, v, chain, err, l, h);
+      if (d != dir) continue;
 #pragma unroll
       for (int c = 0; c < 5; c++) {
-        const T sd = sm.sig[ms][d][c][my][mx];
-        uf[c] = side ? u[c] + T(0.5) * sd : u[c] - T(0.5) * sd;
+        lo[c] = l[c];
+        hi[c] = h[c];
       }
-      e.c2p(uf, out);
-      return;
-    }
-#pragma unroll
-    for (int c = 0; c < 5; c++) {
-      const T v = M2C_VV(s0, c, my + 1, mx + 1);
-      const T sd = sm.sig[ms][d][c][my][mx];
-      out[c] = rev ? v : (side ? v + T(0.5) * sd : v - T(0.5) * sd);
     }
   };
 
-  // (3) flux across the face between mask-region cells L (plane pL) and
-  // R = L + e_d (plane pR): the flux seen by the left cell (F). F2 (the right
-  // cell's) equals F except at NUMERICAL interface faces, where the update
-  // phase forms it.
-  auto face_flux = [&](int d, int pL, int mxL, int myL, int pR, int mxR, int myR, T* F, T* F2) {
-    const int sL = slot4(pL), sR = slot4(pR);
-    const bool rL = sm.real[sL][myL + 1][mxL + 1], rR = sm.real[sR][myR + 1][mxR + 1];
-    if (!rL && !rR) {
-#pragma unroll
-      for (int c = 0; c < 5; c++) { F[c] = T(0); F2[c] = T(0); }
-      return;
+  // Flux across the low face along d of the cell at (cx, cy) of plane p (the
+  // face's right cell), as its left cell sees it. VL, VR: the two cells' face
+  // states, rL, rR: whether they are real (a ghost's is formed here). At a
+  // NUMERICAL interface face the right cell forms its own flux in its update.
+  auto face_flux = [&](auto pin, int d, int p, int cx, int cy, bool rL, bool rR, T* VL, T* VR, T* F) {
+    const int ox = d == 0 ? 1 : 0, oy = d == 1 ? 1 : 0;
+    const int sR = slot_of(p), sL = d == 2 ? slot_of(p - 1) : sR;
+    int idL = 0, idR = 0;
+    if (MULTI) {
+      if (rL) idL = sm.id[sL].v[cy - oy][cx - ox + 12];
+      if (rR) idR = sm.id[sR].v[cy][cx + 12];
+      if (!rL) idL = idR;
+      if (!rR) idR = idL;
     }
-    T VL[5], VR[5];
-    const uint8_t idL = sm.ids[sL][myL + 1][mxL + 1], idR = sm.ids[sR][myR + 1][mxR + 1];
+    // Boundary face state built from the interior neighbour's face state
+    // (Reconstructor.cpp:822-875), and from the ghost cell's where that
+    // needs clipping (CheckReconstructedStates, 3279-3318).
+    if (!rL || !rR) {
+      T im[5], gc[5];
+#pragma unroll
+      for (int c = 0; c < 5; c++) im[c] = rR ? sm.v[sR].v[c][cy][cx] : sm.v[sL].v[c][cy - oy][cx - ox];
+      const int bc = g.bc[2 * d + (rR ? 0 : 1)];
+      ghost_cell(g, d, bc, im, gc);
+      ghost_face(bc, d, rR ? VR : VL, gc, eos_of<T, MULTI, SG>(a.s, idR), rR ? VL : VR);
+    }
     // a face cut by an embedded surface (interior faces only) takes the wall
     // branch, which the reference tests before the material-interface one
     bool wall = false;
-    long long offW = 0;
-    if (WALLS && rL && rR) {
-      const int gi = wrap_index(i0 + mxR - 1, g.nx), gj = wrap_index(j0 + myR - 1, g.ny);
-      offW = (long long)wrap_index(pR, g.nz) * g.plane + (long long)gj * g.px + gi;
-      wall = (a.wall.mask[offW] >> d) & 1;
+    long long offR = 0;
+    if (MULTI && rL && rR && (WALLS || idL != idR)) {
+      offR = (long long)wrap_index(p, g.nz) * g.plane + (long long)wrap_index(j0 + cy - 2, g.ny) * g.px +
+             wrap_index(i0 + cx - 4, g.nx);
+      if (WALLS) wall = (a.wall.mask[offR] >> d) & 1;
     }
-    // face pass: only the faces whose states a pre-pass solves from
-    const bool fp_iface = MULTI && a.iface.faces_out && idL != idR;
-    const bool fp_wall = WALLS && a.wall.faces_out && wall;
-    if (MULTI && (a.iface.faces_out || (WALLS && a.wall.faces_out)) && !fp_iface && !fp_wall) {
-#pragma unroll
-      for (int c = 0; c < 5; c++) { F[c] = T(0); F2[c] = T(0); }
-      return;
-    }
-    if (rL) cell_face(pL, mxL, myL, d, 1, VL);
-    if (rR) cell_face(pR, mxR, myR, d, 0, VR);
-    if (!rL) {  // low-side boundary face
-      T gc[5];
-#pragma unroll
-      for (int c = 0; c < 5; c++) gc[c] = M2C_VV(sL, c, myL + 1, mxL + 1);
-      ghost_face(g.bc[2 * d], d, VR, gc, eos_of<T, MULTI>(a.s, idL), VL);
-    }
-    if (!rR) {  // high-side boundary face
-      T gc[5];
-#pragma unroll
-      for (int c = 0; c < 5; c++) gc[c] = M2C_VV(sR, c, myR + 1, mxR + 1);
-      ghost_face(g.bc[2 * d + 1], d, VL, gc, eos_of<T, MULTI>(a.s, idR), VR);
-    }
-    int err = ERR_NONE;
-    if (fp_iface || fp_wall) {  // face pass: the interface or cut faces' states only
-#pragma unroll
-      for (int c = 0; c < 5; c++) { F[c] = T(0); F2[c] = T(0); }
-      const int gi = wrap_index(i0 + mxR - 1, g.nx), gj = wrap_index(j0 + myR - 1, g.ny);
-      const int gk = wrap_index(pR, g.nz);
-      const long long offR = (long long)gk * g.plane + (long long)gj * g.px + gi;
+    if (face_pass) {  // the states a pre-pass solves from, and nothing else
       for (int q = 0; q < 2; q++) {
-        if (q == 0 ? !fp_iface : !fp_wall) continue;
+        if (q == 0 ? !(a.iface.faces_out && idL != idR) : !(WALLS && a.wall.faces_out && wall)) continue;
         const int slot = q == 0 ? a.iface.slot[offR] : a.wall.slot[offR];
         double* o = (q == 0 ? a.iface.faces_out : a.wall.faces_out) + ((long long)slot * 3 + d) * 10;
 #pragma unroll
@@ -846,129 +746,50 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
       // no surface cuts carries none (SpaceOperator.cpp:2441-2483, 2537-2551);
       // the right cell of a cut face forms its own flux in its update
 #pragma unroll
-      for (int c = 0; c < 5; c++) { F[c] = T(0); F2[c] = T(0); }
+      for (int c = 0; c < 5; c++) F[c] = T(0);
       return;
     }
+    int err = ERR_NONE;
+    const Eos<T>* e = &eos_of<T, MULTI, SG>(a.s, idR);  // the right cell's EOS, as the reference's face loop
     if (MULTI && (wall || idL != idR)) {
       // Material interface (SpaceOperator.cpp:2486-2542): two one-sided fluxes
       // against the exact Riemann star states, or LLF across the interface.
-      // Wall (2438-2484, CONSTANT reconstruction at the wall): the left
-      // cell's flux against its one-sided star state.
+      // Wall (2438-2484): the left cell's flux against its one-sided star state.
       const IfaceView& iv = a.iface;
-      T WL[5], WR[5];
       if (wall ? !a.wall.linear : iv.mp_recon == 0) {  // constant reconstruction: cell-centred states
 #pragma unroll
         for (int c = 0; c < 5; c++) {
-          WL[c] = M2C_VV(sL, c, myL + 1, mxL + 1);
-          WR[c] = M2C_VV(sR, c, myR + 1, mxR + 1);
+          VL[c] = sm.v[sL].v[c][cy - oy][cx - ox];
+          VR[c] = sm.v[sR].v[c][cy][cx];
         }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 5; c++) { WL[c] = VL[c]; WR[c] = VR[c]; }
       }
       if (!wall && iv.mp_flux == 2) {
-        err = flux_llf2(eos_of<T, MULTI>(a.s, idL), eos_of<T, MULTI>(a.s, idR), d, WL, WR, F);
-#pragma unroll
-        for (int c = 0; c < 5; c++) F2[c] = F[c];
-      } else {
-        // the right cell's index carries the slot of its low faces
-        const int gi = wrap_index(i0 + mxR - 1, g.nx), gj = wrap_index(j0 + myR - 1, g.ny);
-        const int gk = wrap_index(pR, g.nz);
-        const int slot = wall ? a.wall.slot[offW] : iv.slot[(long long)gk * g.plane + (long long)gj * g.px + gi];
-        const long long base = ((long long)slot * 3 + d) * 5;
-        if (!wall && iv.mp_flux == 0) {  // Godunov flux of the state at xi = 0
-          T Vm[5];
-#pragma unroll
-          for (int c = 0; c < 5; c++) Vm[c] = T(iv.Vmid[base + c]);
-          phys_flux(eos_of<T, MULTI>(a.s, iv.midid[slot * 3 + d]), d, Vm, F);
-#pragma unroll
-          for (int c = 0; c < 5; c++) F2[c] = F[c];
-        } else {
-          const double* src = wall ? a.wall.Vsm : iv.Vsm;
-          T Sm[5];
-#pragma unroll
-          for (int c = 0; c < 5; c++) Sm[c] = T(src[base + c]);
-          // the right cell's flux against its own star state is formed in its update
-          err = flux_of<T, FLUX>(eos_of<T, MULTI>(a.s, idL), d, WL, Sm, delta, F);
-        }
+        err = flux_llf2(eos_of<T, MULTI, SG>(a.s, idL), eos_of<T, MULTI, SG>(a.s, idR), d, VL, VR, F);
+        if (err) report(a.err, err, -1, where + 2);
+        return;
       }
-    } else {
-      // same material: flux with the right cell's EOS, as the reference's
-      // face loop does (myid = id of the right cell)
-      err = flux_of<T, FLUX>(eos_of<T, MULTI>(a.s, rR ? idR : idL), d, VL, VR, delta, F);
+      const int slot = wall ? a.wall.slot[offR] : iv.slot[offR];  // held by the right cell
+      const long long base = ((long long)slot * 3 + d) * 5;
+      if (!wall && iv.mp_flux == 0) {  // Godunov flux of the state at xi = 0
+        T Vm[5];
 #pragma unroll
-      for (int c = 0; c < 5; c++) F2[c] = F[c];
+        for (int c = 0; c < 5; c++) Vm[c] = T(iv.Vmid[base + c]);
+        phys_flux(eos_of<T, MULTI, SG>(a.s, iv.midid[slot * 3 + d]), d, Vm, F);
+        return;
+      }
+      const double* src = wall ? a.wall.Vsm : iv.Vsm;
+#pragma unroll
+      for (int c = 0; c < 5; c++) VR[c] = T(src[base + c]);
+      e = &eos_of<T, MULTI, SG>(a.s, idL);
     }
+    err = flux_of<T, FLUX, decltype(pin)::value>(*e, d, VL, VR, delta, F);
     if (err) report(a.err, err, -1, where + 2);
   };
 
-  // (3a) the faces of plane m owned by this thread: the x face left of its
-  // cell, the y face below it (if do_xy) and the z face m+1/2 above it; one
-  // call site, so the flux code is inlined once.
-  auto faces = [&](int m, bool do_xy) {
-    const int zs = (m + 1) & 1;
-#pragma unroll 1
-    for (int k = do_xy ? 0 : 2; k < 3; k++) {
-      const int d = k;
-      const int mxL = k == 0 ? tx : tx + 1, myL = k == 1 ? ty : ty + 1;
-      const int pR = k == 2 ? m + 1 : m;
-      T* dst = k == 0 ? &sm.fx[0][ty * (TX + 1) + tx] : (k == 1 ? &sm.fy[0][ty * TX + tx] : &sm.fz[zs][0][ty * TX + tx]);
-      const int stride = k == 0 ? S::NFX : (k == 1 ? S::NFY : S::NFZ);
-      T F[5], F2[5];
-      face_flux(d, m, mxL, myL, pR, tx + 1, ty + 1, F, F2);
-#pragma unroll
-      for (int c = 0; c < 5; c++) dst[c * stride] = F[c];
-    }
-  };
-
-  // (2) + (3b) one phase: slopes and revert bits of plane p (do_mask): the
-  // tile's cells, one per thread, then the halo cells in their single
-  // direction; and the tile's right x faces and top y faces of plane mf
-  // (do_bf), whose cells' slopes are complete since the previous plane.
-  // Spreading the halo cells and those faces over the threads that have no
-  // second item keeps the phase at about one cell and a third per thread.
-  auto mask_and_edge_faces = [&](int p, bool do_mask, int mf, bool do_bf) {
-    constexpr int NH = CONS ? S::MX * S::MY - NT : 2 * (TX + TY);  // halo items
-    constexpr int NB = TX + TY;                                     // edge faces
-    for (int q = tid; q < NT + NH + NB; q += NT) {
-      if (q < NT + NH) {
-        if (!do_mask) continue;
-        const int r = q - NT;
-        int mx = tx + 1, my = ty + 1, dh = 0;
-        if (r < 0) {
-          // a cell of the tile
-        } else if (CONS) {  // the ring of the mask region: bottom row, top row, then the two side columns
-          if (r < S::MX) { mx = r; my = 0; }
-          else if (r < 2 * S::MX) { mx = r - S::MX; my = S::MY - 1; }
-          else { const int r2 = r - 2 * S::MX; mx = (r2 & 1) ? S::MX - 1 : 0; my = 1 + (r2 >> 1); }
-        } else if (r < 2 * TY) {  // x-halo columns (mx = 0, TX + 1)
-          mx = r < TY ? 0 : TX + 1;
-          my = (r < TY ? r : r - TY) + 1;
-        } else {                  // y-halo rows (my = 0, TY + 1)
-          const int r2 = r - 2 * TY;
-          mx = (r2 < TX ? r2 : r2 - TX) + 1;
-          my = r2 < TX ? 0 : TY + 1;
-          dh = 1;
-        }
-        mask_cell(p, mx, my, r < 0, dh);
-      } else {
-        if (!do_bf) continue;
-        const int r = q - NT - NH;
-        const bool xf = r < TY;  // x face right of the tile's last column (row r), else
-                                 // y face above its top row (column r - TY)
-        const int fx = r - TY;
-        T F[5], F2[5];
-        face_flux(xf ? 0 : 1, mf, xf ? TX : fx + 1, xf ? r + 1 : TY, mf, xf ? TX + 1 : fx + 1, xf ? r + 1 : TY + 1, F,
-                  F2);
-        T* dst = xf ? &sm.fx[0][r * (TX + 1) + TX] : &sm.fy[0][TY * TX + fx];
-        const int stride = xf ? S::NFX : S::NFY;
-#pragma unroll
-        for (int c = 0; c < 5; c++) dst[c * stride] = F[c];
-      }
-    }
-  };
-
-  double dtmin_local = 1.0e300;
+  // per-thread CFL extremes: the largest |u| + c seen against each axis'
+  // current width (dx / max is the smallest quotient, rounding being
+  // monotonic), turned into a time step when a width changes
+  double lmax[3] = {0.0, 0.0, 0.0}, dtmin_local = 1.0e300;
   int clipped_local = 0;
   const int tiles = a.ntx * a.nty;
 
@@ -983,33 +804,70 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
     const int ke = (int)min((long long)g.nz, kb + (uend - u));
     u += ke - kb;
     const int tyi = t2 / a.ntx, txi = t2 - tyi * a.ntx;
+    __syncthreads();  // the previous segment's last reads (and the mbarriers' initialisation)
     i0 = txi * TX;
     j0 = tyi * TY;
-    const int gi = i0 + tx, gj = j0 + ty;
-    const bool own = gi < g.nx && gj < g.ny;
-    double dxi = 0, dyj = 0;
+    pbase = kb - 2;
+    fcl = i0 == 0 ? 2 : 0;
+    frl = j0 == 0 ? 2 : 0;
+    fncol = (fcl + max(0, min(i0 + TX + 2 - g.nx, 2))) * S::RY;
+    fn = fncol + (frl + max(0, min(j0 + TY + 2 - g.ny, 2))) * S::RX;
+    const int gi = i0 + lane, gj = j0 + row;
+    const bool own = !edge && gi < g.nx && gj < g.ny;
+    // Cells this thread reconstructs, and the faces it owns. A row's own
+    // cells take all directions; a wrapped cell beyond a periodic boundary
+    // inside the tile only the one whose face needs it.
+    const bool inx = gi < g.nx, iny = gj < g.ny;
+    const bool sx_act = own || (xper && !edge && gi == g.nx && iny), sy_act = own || (yper && !edge && gj == g.ny && inx);
+    const bool fx_act = !edge && iny && gi <= g.nx, fy_act = !edge && inx && gj <= g.ny;
+    // Extra items: states of the x-halo columns (lanes 0-15 the low one,
+    // 16-31 the high one), of the low and the high halo row; fluxes of the
+    // tile's high x and y faces.
+    const int er = lane & 15, ehi = lane >> 4;
+    const bool er_in = er < TY && j0 + er < g.ny;
+    const bool hx_act = er_in && (ehi ? (i0 + TX < g.nx || (xper && i0 + TX == g.nx)) : (i0 > 0 || xper));
+    const bool ylo_act = inx && (j0 > 0 || yper), yhi_act = inx && (j0 + TY < g.ny || (yper && j0 + TY == g.ny));
+    const bool hfx_act = er_in && ehi && i0 + TX <= g.nx, hfy_act = inx && j0 + TY <= g.ny;
+    // real cells left and right of this thread's low x (bits 0, 1) and y (bits 2, 3) face
+    const int lr = (gi > 0 || xper ? 1 : 0) | (inx || xper ? 2 : 0) | (gj > 0 || yper ? 4 : 0) | (iny || yper ? 8 : 0);
+    // first item of this warp's loops (its own directions and faces are 0, 1, 2)
+    const int a_first = EW ? (edge ? -3 : 0) : (row < 3 ? -1 : 0), a_end = edge ? 0 : 3;
+    const int b_first = EW ? (edge ? -2 : 0) : (row == 3 || row == 4 ? -1 : 0);
+    double dxi = 0, dyj = 0, dzc = 0, inv_mvol = 0, ax = 0, ay = 0;
     if (own) { dxi = g.dx[gi]; dyj = g.dy[gj]; }
+    const double az = dxi * dyj;
+    float axf = 0.f, ayf = 0.f;
+    const float azf = float(az);
+    // cell offsets fit 32 bits: 2^32 cells would not fit the device
+    const unsigned plane32 = unsigned(g.plane), offc = unsigned(gj) * unsigned(g.px) + unsigned(gi);
 
-    // pipeline prologue: planes kb-2 and kb-1 committed, plane kb in flight
-    // (a plane copy that never lands stops the CTA, all threads together)
-    tile_setup();
-    __syncthreads();
-    issue_plane(kb - 2);
-    bool landed = wait_plane(kb - 2);
-    commit_plane(kb - 2);
+    // pipeline prologue: RING planes in flight, the halos iteration kb-1 reads ready
+    bool landed = true;
+    if (copier)
+      for (int p = kb - 2; p < kb - 2 + RING; p++)
+        if (p <= ke + 1 && real_plane(p)) issue_plane(p);
+    for (int p = kb - 2; p <= kb; p++) {
+      if (!real_plane(p)) continue;
+      landed = wait_plane(p) && landed;
+      if (landed && (CONS || p > kb - 2)) fix_plane(p);
+    }
     if (__syncthreads_or(!landed)) return;
-    issue_plane(kb - 1);
-    landed = wait_plane(kb - 1);
-    commit_plane(kb - 1);
-    if (__syncthreads_or(!landed)) return;
-    issue_plane(kb);
-    for (int m = kb - 2; m < ke; m++) {
-      landed = wait_plane(m + 2);
-      commit_plane(m + 2);
-      if (__syncthreads_or(!landed)) return;
-      if (m + 3 <= ke + 1) issue_plane(m + 3);  // in flight during the work below
-      if (m >= kb && own) {  // the update's FP64 inputs of plane m into L1 while the faces are computed
-        const long long offp = (long long)m * g.plane + (long long)gj * g.px + gi;
+
+    T pz[5];             // high z face state of plane p-1
+    double part[5];      // FP64: flux sum of plane p-1 without its face p-1/2
+    T dxy[5], hl[5];     // mixed: x and y flux differences of plane p-1, flux of face p-3/2
+    int idprev = 0;      // material of plane p-1
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      pz[c] = dxy[c] = hl[c] = T(0);
+      part[c] = 0.0;
+    }
+    for (int p = kb - 1; p <= ke; p++) {
+      const bool rp = real_plane(p), in = p >= kb && p < ke;
+      const int s0 = slot_of(p);
+      // ---- A(p)
+      if (p > kb && own && !face_pass) {  // the update's FP64 inputs of plane p-1 into L1
+        const unsigned offp = unsigned(p - 1) * plane32 + offc;
 #pragma unroll
         for (int c = 0; c < 5; c++) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.Vn[c] + offp));
         if (a.stage != 1) {
@@ -1017,213 +875,342 @@ __global__ void __launch_bounds__(TX * TY, StageOcc<T>::value) stage_kernel(cons
           for (int c = 0; c < 5; c++) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.Us[c] + offp));
         }
       }
-      mask_and_edge_faces(m + 1, m + 1 >= kb - 1 && !plane_is_ghost(m + 1), m, m >= kb);
-      __syncthreads();
-      if (m >= kb - 1) faces(m, m >= kb);
-      __syncthreads();
-      if (m < kb || !own || (MULTI && (a.iface.faces_out || (WALLS && a.wall.faces_out)))) continue;
-      // (4) residual + RK update of plane m
-      const double dzk = g.dz[m];
-      const double ax = dyj * dzk, ay = dxi * dzk, az = dxi * dyj;
-      const float axf = float(ax), ayf = float(ay), azf = float(az);
-      const double vol = dxi * dyj * dzk;
-      // Vec5D::operator/= multiplies by the reciprocal (Vector5D.h:172-181)
-      const double inv_mvol = 1.0 / (-vol);
-      const long long off = (long long)m * g.plane + (long long)gj * g.px + gi;
-      const uint8_t id = MULTI ? a.id[off] : 0;
-      if (WALLS && id == a.s.nmat) {
-        // inactive: no residual (every face gives it a zero flux), and
-        // VarFcnDummy's fixed states after every stage (VarFcnDummy.h:44-57)
-        if (a.Ro[0]) {
+      T pzn[5];
 #pragma unroll
-          for (int c = 0; c < 5; c++) a.Ro[c][off] = 0.0 * inv_mvol;
-          continue;
-        }
-        const double Vd[5] = {a.s.dummy[0], 0.0, 0.0, 0.0, a.s.dummy[1]};
-        if (a.final_stage) {
+      for (int c = 0; c < 5; c++) pzn[c] = T(0);
+      int idp = 0;
+      if (rp) {
+        int err = ERR_NONE;
+        bool chain = false;
+        auto item = [&](int it) {
+          const int k = EW ? it + 3 : row;  // which extra item (it < 0)
+          const int d = it >= 0 ? it : (k == 0 ? 0 : 1);
+          const int cx = it < 0 && k == 0 ? (ehi ? TX + 4 : 3) : lane + 4;
+          const int cy = it >= 0 ? row + 2 : (k == 0 ? er + 2 : (k == 1 ? 1 : TY + 2));
+          if (it >= 0 ? !(it == 0 ? sx_act : (it == 1 ? sy_act : own))
+                      : !(in && (k == 0 ? hx_act : (k == 1 ? ylo_act : yhi_act))))
+            return;
+          T v[5], lo[5], hi[5];
 #pragma unroll
-          for (int c = 0; c < 5; c++) a.Vo[c][off] = Vd[c];
-          if (a.Vfo[0]) {
+          for (int c = 0; c < 5; c++) v[c] = sm.v[s0].v[c][cy][cx];
+          const int id = MULTI ? sm.id[s0].v[cy][cx + 12] : 0;
+          const Eos<T>& e = eos_of<T, MULTI, SG>(a.s, id);
+          int bad = ERR_NONE;
+          if (WALLS && id == a.s.nmat) {  // inactive: constant reconstruction, no checks
 #pragma unroll
-            for (int c = 0; c < 5; c++) a.Vfo[c][off] = float(Vd[c]);
+            for (int c = 0; c < 5; c++) lo[c] = hi[c] = v[c];
+          } else if constexpr (CONS) {
+            cons_states(d, p, cx, cy, id, e, v, bad, lo, hi);
+          } else {
+            if (it <= 0 || !own) chain = false;  // another cell than in the last iteration
+            face_states(d, p, cx, cy, id, e, v, chain, bad, lo, hi);
           }
+          if (it >= 0 && bad) err = bad;
+          // of a low halo only the high state is read, of a high one only the low state
+          const bool put_lo = it >= 0 || (k == 0 ? ehi : k == 2);
+          T* plo = d == 0 ? &sm.lox[0][cy - 2][cx - 4] : (d == 1 ? &sm.loy[0][cy - 2][lane] : &sm.loz[0][row][lane]);
+          T* phi = d == 0 ? &sm.hix[0][cy - 2][cx - 3] : &sm.hiy[0][cy - 1][lane];
+          const int st = d == 0 ? XS : (d == 1 ? YS : ZS);
+          if (put_lo) {
+#pragma unroll
+            for (int c = 0; c < 5; c++) plo[c * st] = lo[c];
+          }
+          if (it == 2) {
+#pragma unroll
+            for (int c = 0; c < 5; c++) pzn[c] = hi[c];
+          } else if (it >= 0 || !put_lo) {
+#pragma unroll
+            for (int c = 0; c < 5; c++) phi[c * st] = hi[c];
+          }
+          if (MULTI && it >= 0) idp = id;
+        };
+        // Own directions unrolled in the one-material kernel (4% off the FP32
+        // stage of a 256^3 box); in the two-material one that spills (3% more).
+        if constexpr (MULTI) {
+#pragma unroll 1
+          for (int it = a_first; it < a_end; it++) item(it);
         } else {
+#pragma unroll 1
+          for (int it = a_first; it < 0; it++) item(it);
+          if (!edge) {
+            item(0);
+            item(1);
+            item(2);
+          }
+        }
+        if (err && own) {
+          const int ka = wrap_index(p, g.nz);
+          report(a.err, err, (int)(((long long)ka * g.ny + gj) * g.nx + gi), where + 1);
+        }
+      }
+      __syncthreads();
+      // ---- B(p): the low x, y and z faces of the cell, last so that F ends as the z flux
+      T F[5];
+#pragma unroll 1
+      for (int it = b_first; it < a_end; it++) {
+        const int k = EW ? it + 2 : row - 3;  // which extra item (it < 0): high x faces, high y faces
+        const int d = it >= 0 ? it : k;
+        if (it >= 0 ? !(it == 0 ? in && fx_act : (it == 1 ? in && fy_act : own && p >= kb))
+                    : !(in && (k == 0 ? hfx_act : hfy_act)))
+          continue;
+        const int cx = it < 0 && k == 0 ? TX + 4 : lane + 4, cy = it >= 0 ? row + 2 : (k == 0 ? er + 2 : TY + 2);
+        const int st = d == 0 ? XS : (d == 1 ? YS : ZS);
+        const int at = d == 0 ? (cy - 2) * (TX + 1) + cx - 4 : (cy - 2) * TX + lane;
+        const T* ph = (d == 0 ? &sm.hix[0][0][0] : &sm.hiy[0][0][0]) + at;
+        const T* pl = (d == 0 ? &sm.lox[0][0][0] : (d == 1 ? &sm.loy[0][0][0] : &sm.loz[0][0][0])) + at;
+        T VL[5], VR[5];
+#pragma unroll
+        for (int c = 0; c < 5; c++) {
+          VL[c] = d == 2 ? pz[c] : ph[c * st];
+          VR[c] = pl[c * st];
+        }
+        const int f2 = it < 0 ? (1 | ((k == 0 ? hx_act : yhi_act) ? 2 : 0))
+                              : (d == 2 ? (real_plane(p - 1) ? 1 : 0) | (rp ? 2 : 0) : lr >> (2 * d));
+        const bool rL = f2 & 1, rR = f2 & 2;
+        // FP32: faces between blocks of 32 x 16 cells, as their left cells
+        // see them, go through a call of their own, whose contraction is the
+        // compiler's (see PIN_MOMENTUM): the mixed path's values stay as they were
+        if (sizeof(T) == 4 && it < 0 && (k == 0 || ((j0 + TY) & 15) == 0))
+          face_flux(std::integral_constant<int, PIN & ~PIN_MOMENTUM>(), k == 0 ? 0 : 1, p, cx, cy, rL, rR, VL, VR, F);
+        else
+          face_flux(std::integral_constant<int, PIN>(), d, p, cx, cy, rL, rR, VL, VR, F);
+        if (d < 2) {
+          T* pf = (d == 0 ? &sm.fx[0][0][0] : &sm.fy[0][0][0]) + at;
+#pragma unroll
+          for (int c = 0; c < 5; c++) pf[c * st] = F[c];
+        }
+      }
+      if (p > kb && own && !face_pass) {
+        // F is the flux of face p-1/2: residual + RK update of plane m
+        const int m = p - 1;
+        const unsigned off = unsigned(m) * plane32 + offc;
+        const int id = idprev;
+        if (WALLS && id == a.s.nmat) {
+          // inactive: no residual (every face gives it a zero flux), and
+          // VarFcnDummy's fixed states after every stage (VarFcnDummy.h:44-57)
+          const double Vd[5] = {a.s.dummy[0], 0.0, 0.0, 0.0, a.s.dummy[1]};
           const double Ud[5] = {a.s.dummy[0], 0.0, 0.0, 0.0, a.s.dummy[0] * a.s.dummy[2]};
 #pragma unroll
           for (int c = 0; c < 5; c++) {
-            a.Uo[c][off] = Ud[c];
-            static_cast<T*>(a.Po[c])[off] = T(Vd[c]);
+            if (a.Ro[0]) {
+              a.Ro[c][off] = 0.0 * inv_mvol;
+            } else if (a.final_stage) {
+              a.Vo[c][off] = Vd[c];
+              if (a.Vfo[0]) a.Vfo[c][off] = float(Vd[c]);
+            } else {
+              a.Uo[c][off] = Ud[c];
+              static_cast<T*>(a.Po[c])[off] = T(Vd[c]);
+            }
           }
-        }
-        continue;
-      }
-      const Eos<double>& e = eos_of<double, MULTI>(a.s, id);
-      double Un[5], Unew[5], Vn[5];
+        } else {
+          const Eos<double>& e = eos_of<double, MULTI, SG>(a.s, id);
+          double Un[5], Unew[5], Vn[5];
 #pragma unroll
-      for (int c = 0; c < 5; c++) Vn[c] = a.Vn[c][off];
-      e.p2c(Vn, Un);
-      if (a.stage == 1) {
+          for (int c = 0; c < 5; c++) Vn[c] = a.Vn[c][off];
+          e.p2c(Vn, Un);
+          if (a.stage == 1) {
 #pragma unroll
-        for (int c = 0; c < 5; c++) Unew[c] = Un[c];
-      } else {
-        double Us[5];
+            for (int c = 0; c < 5; c++) Unew[c] = Un[c];
+          } else {
+            double Us[5];
 #pragma unroll
-        for (int c = 0; c < 5; c++) Us[c] = a.Us[c][off];
-        if (us_clip) {
-          double Vs[5];
-          e.c2p(Us, Vs);
-          e.clip(Vs);
-          e.p2c(Vs, Us);
-        }
+            for (int c = 0; c < 5; c++) Us[c] = a.Us[c][off];
+            if (us_clip) {
+              double Vs[5];
+              e.c2p(Us, Vs);
+              e.clip(Vs);
+              e.p2c(Vs, Us);
+            }
 #pragma unroll
-        for (int c = 0; c < 5; c++) Unew[c] = a.a_prev * Us[c] + a.a_un * Un[c];
-      }
-      const int fxl = ty * (TX + 1) + tx, fyl = ty * TX + tx, fzc = ty * TX + tx;
-      const int zl = m & 1, zr = (m + 1) & 1;
-      // Low faces that are material interfaces under the NUMERICAL interface
-      // flux: this cell's flux is its EOS's numerical flux between the right
-      // star state and its own cell-centred state (SpaceOperator.cpp:2499-2542).
-      // Low faces cut by an embedded surface likewise take this cell's flux
-      // against its one-sided star state (SpaceOperator.cpp:2462-2478).
-      T F2[3][5];
-      bool ifc[3] = {false, false, false};
-      if constexpr (MULTI) {
-        const uint8_t wm = WALLS ? a.wall.mask[off] : 0;
-        const bool num = a.iface.mp_flux == 1;  // set only with interface slots (two-material contexts)
-        if (num || wm) {
-          const int sc = slot4(m), lx = tx + 2, ly = ty + 2;
-          const uint8_t me = sm.ids[sc][ly][lx];
-          ifc[0] = (wm & 1) || (num && me != sm.ids[sc][ly][lx - 1]);
-          ifc[1] = (wm & 2) || (num && me != sm.ids[sc][ly - 1][lx]);
-          ifc[2] = (wm & 4) || (num && me != sm.ids[slot4(m - 1)][ly][lx]);
-          if (ifc[0] || ifc[1] || ifc[2]) {
-            const int islot = num ? a.iface.slot[off] : 0;
-            const int wslot = wm ? a.wall.slot[off] : 0;
-            for (int d = 0; d < 3; d++) {
-              if (!ifc[d]) continue;
-              const bool w = (wm >> d) & 1;
-              // this cell's side of the face: its cell-centred state, or its
-              // reconstructed state on that face (vl) under LINEAR interface
-              // reconstruction
-              T W[5];
-              if (w ? a.wall.linear : a.iface.mp_recon) {
-                cell_face(m, tx + 1, ty + 1, d, 0, W);
+            for (int c = 0; c < 5; c++) Unew[c] = a.a_prev * Us[c] + a.a_un * Un[c];
+          }
+#pragma unroll
+          for (int c = 0; c < 5; c++) {
+            double f;
+            if constexpr (sizeof(T) == 8) f = part[c] + double(F[c]) * az;
+            else f = double(dxy[c] + (F[c] - hl[c]) * azf);
+            if (a.visc.fr[0]) {
+              // viscous fluxes (ViscosityOperator::AddDiffusionFluxes), added to
+              // the flux sum in its cell order: this cell's low x, y, z faces,
+              // then the low faces of its +x, +y, +z neighbours
+              if (c == 0) {
+                f = f + 0.0; f = f + 0.0; f = f + 0.0;
+                f = f - 0.0; f = f - 0.0; f = f - 0.0;
               } else {
-#pragma unroll
-                for (int c = 0; c < 5; c++) W[c] = M2C_VV(sc, c, ly, lx);
+                const long long Sv = a.visc.nf[0], cc = (long long)(c - 1) * Sv;
+                const long long fxi = ((long long)m * g.ny + gj) * (g.nx + 1) + gi;
+                const long long fyi = ((long long)m * (g.ny + 1) + gj) * g.nx + gi;
+                const long long fzi = ((long long)m * g.ny + gj) * g.nx + gi;
+                f = f + a.visc.fr[0][cc + fxi];
+                f = f + a.visc.fr[1][cc + fyi];
+                f = f + a.visc.fr[2][cc + fzi];
+                f = f - a.visc.fl[0][cc + fxi + 1];
+                f = f - a.visc.fl[1][cc + fyi + g.nx];
+                f = f - a.visc.fl[2][cc + fzi + (long long)g.ny * g.nx];
               }
-              const long long base = ((long long)(w ? wslot : islot) * 3 + d) * 5;
-              const double* src = w ? a.wall.Vsp : a.iface.Vsp;
-              T Sp[5];
+            }
+            if (c == 4 && a.visc.fh[0]) {
+              // heat fluxes (HeatDiffusionOperator::AddDiffusionFluxes, after the
+              // viscous ones), energy only, in the same cell order
+              const long long fxi = ((long long)m * g.ny + gj) * (g.nx + 1) + gi;
+              const long long fyi = ((long long)m * (g.ny + 1) + gj) * g.nx + gi;
+              const long long fzi = ((long long)m * g.ny + gj) * g.nx + gi;
+              f = f + a.visc.fh[0][fxi];
+              f = f + a.visc.fh[1][fyi];
+              f = f + a.visc.fh[2][fzi];
+              f = f - a.visc.fh[0][fxi + 1];
+              f = f - a.visc.fh[1][fyi + g.nx];
+              f = f - a.visc.fh[2][fzi + (long long)g.ny * g.nx];
+            }
+            const double R = f * inv_mvol;
+            if (a.Ro[0]) a.Ro[c][off] = R;
+            Unew[c] = Unew[c] + bdt * R;
+          }
+          if (!a.Ro[0]) {
+            double V[5];
+            e.c2p(Unew, V);
+            const bool clipped = e.clip(V);
+            clipped_local |= clipped ? 1 : 0;
+            if (e.bad(V))
+              report(a.err, ERR_STATE, (int)((long long)m * g.ny * g.nx + (long long)gj * g.nx + gi), where + 3);
+            if (a.final_stage) {
 #pragma unroll
-              for (int c = 0; c < 5; c++) Sp[c] = T(src[base + c]);
-              const int err2 = flux_of<T, FLUX>(eos_of<T, MULTI>(a.s, me), d, Sp, W, delta, F2[d]);
-              if (err2) report(a.err, err2, -1, where + 2);
+              for (int c = 0; c < 5; c++) a.Vo[c][off] = V[c];
+              if (a.Vfo[0]) {
+#pragma unroll
+                for (int c = 0; c < 5; c++) a.Vfo[c][off] = float(V[c]);
+              }
+              const double ee = e.energy(V[0], V[4]);
+              const double c2 = e.c2(V[0], ee);
+              if (c2 < 0.0) report(a.err, ERR_SOUND, (int)off, where + 4);
+              const double cs = sqrt(c2);
+#pragma unroll
+              for (int d = 0; d < 3; d++) lmax[d] = smax(lmax[d], fabs(V[1 + d]) + cs);
+            } else {
+#pragma unroll
+              for (int c = 0; c < 5; c++) a.Uo[c][off] = Unew[c];
+              // the next stage's input: clip(C2P(U_new)), as it would recompute it
+#pragma unroll
+              for (int c = 0; c < 5; c++) static_cast<T*>(a.Po[c])[off] = T(V[c]);
             }
           }
         }
       }
-#pragma unroll
-      for (int c = 0; c < 5; c++) {
-        // low faces: the flux this cell sees as the right-hand cell
-        // (SpaceOperator.cpp:2555-2556, 2683-2684, 2810-2811)
-        const T fl = ifc[0] ? F2[0][c] : sm.fx[c][fxl];
-        const T gl = ifc[1] ? F2[1][c] : sm.fy[c][fyl];
-        const T hl = ifc[2] ? F2[2][c] : sm.fz[zl][c][fzc];
-        double f;
-        if constexpr (sizeof(T) == 8) {
-          // FP64: the reference's order, 0 - Fl A - Gl A - Hl A + Fr A + Gr A + Hr A
-          f = 0.0;
-          f = f - fl * ax;
-          f = f - gl * ay;
-          f = f - hl * az;
-          f = f + double(sm.fx[c][fxl + 1]) * ax;
-          f = f + double(sm.fy[c][fyl + TX]) * ay;
-          f = f + double(sm.fz[zr][c][fzc]) * az;
-        } else {
-          // mixed: FP32 accumulation of the flux differences (the difference
-          // of two nearby FP32 fluxes is exact), one conversion per component
-          f = double((sm.fx[c][fxl + 1] - fl) * axf + (sm.fy[c][fyl + TX] - gl) * ayf +
-                     (sm.fz[zr][c][fzc] - hl) * azf);
+      // the halo of the plane after next
+      if (p + 2 <= ke + 1 && real_plane(p + 2)) {
+        landed = wait_plane(p + 2);
+        if (landed) fix_plane(p + 2);
+      }
+      if (__syncthreads_or(!landed)) return;
+      // ---- C(p)
+      if (copier && p + RING - 1 <= ke + 1 && real_plane(p + RING - 1)) issue_plane(p + RING - 1);
+      if (in && own && !face_pass) {
+        const double dzk = g.dz[p];
+        if (dzk != dzc) {
+          ax = dyj * dzk;
+          ay = dxi * dzk;
+          axf = float(ax);
+          ayf = float(ay);
+          if (dzc != 0.0) dtmin_local = smin(dtmin_local, dzc / lmax[2]);
+          lmax[2] = 0.0;
+          dzc = dzk;
+          const double vol = dxi * dyj * dzk;
+          // Vec5D::operator/= multiplies by the reciprocal (Vector5D.h:172-181)
+          inv_mvol = 1.0 / (-vol);
         }
-        if (a.visc.fr[0]) {
-          // viscous fluxes (ViscosityOperator::AddDiffusionFluxes), added to
-          // the flux sum in its cell order: this cell's low x, y, z faces,
-          // then the low faces of its +x, +y, +z neighbours
-          if (c == 0) {
-            f = f + 0.0; f = f + 0.0; f = f + 0.0;
-            f = f - 0.0; f = f - 0.0; f = f - 0.0;
-          } else {
-            const long long S = a.visc.nf[0], cc = (long long)(c - 1) * S;
-            const long long fxi = ((long long)m * g.ny + gj) * (g.nx + 1) + gi;
-            const long long fyi = ((long long)m * (g.ny + 1) + gj) * g.nx + gi;
-            const long long fzi = ((long long)m * g.ny + gj) * g.nx + gi;
-            f = f + a.visc.fr[0][cc + fxi];
-            f = f + a.visc.fr[1][cc + fyi];
-            f = f + a.visc.fr[2][cc + fzi];
-            f = f - a.visc.fl[0][cc + fxi + 1];
-            f = f - a.visc.fl[1][cc + fyi + g.nx];
-            f = f - a.visc.fl[2][cc + fzi + (long long)g.ny * g.nx];
+        // Low faces, the flux this cell sees as the right-hand cell
+        // (SpaceOperator.cpp:2555-2556, 2683-2684, 2810-2811). Low faces that
+        // are material interfaces under the NUMERICAL interface flux: this
+        // cell's flux is its EOS's numerical flux between the right star state
+        // and its own cell-centred state (SpaceOperator.cpp:2499-2542), or
+        // under LINEAR interface reconstruction its reconstructed state. Low
+        // faces cut by an embedded surface likewise take this cell's flux
+        // against its one-sided star state (SpaceOperator.cpp:2462-2478).
+        T FL[3][5];
+#pragma unroll
+        for (int c = 0; c < 5; c++) {
+          FL[0][c] = sm.fx[c][row][lane];
+          FL[1][c] = sm.fy[c][row][lane];
+          FL[2][c] = F[c];
+        }
+        if constexpr (MULTI) {
+          const unsigned off = unsigned(p) * plane32 + offc;
+          const int wm = WALLS ? a.wall.mask[off] : 0;
+          int fm = wm;
+          if (a.iface.mp_flux == 1) {  // set only with interface slots (two-material contexts)
+            fm |= (idp != sm.id[s0].v[row + 2][lane + 15] ? 1 : 0) | (idp != sm.id[s0].v[row + 1][lane + 16] ? 2 : 0) |
+                  (real_plane(p - 1) && idp != idprev ? 4 : 0);
+          }
+          if (fm) {
+            auto own_side = [&](int d) {
+              if (!((fm >> d) & 1)) return;
+              const bool w = (wm >> d) & 1;
+              const T* ps = (w ? a.wall.linear : a.iface.mp_recon)
+                                ? (d == 0 ? &sm.lox[0][row][lane] : (d == 1 ? &sm.loy[0][row][lane] : &sm.loz[0][row][lane]))
+                                : &sm.v[s0].v[0][row + 2][lane + 4];
+              const int st = (w ? a.wall.linear : a.iface.mp_recon) ? (d == 0 ? XS : (d == 1 ? YS : ZS)) : CS;
+              const long long sl = w ? a.wall.slot[off] : a.iface.slot[off];
+              const double* src = (w ? a.wall.Vsp : a.iface.Vsp) + (sl * 3 + d) * 5;
+              T W[5], Sp[5], F2[5];
+#pragma unroll
+              for (int c = 0; c < 5; c++) {
+                W[c] = ps[c * st];
+                Sp[c] = T(src[c]);
+              }
+              const int err2 = flux_of<T, FLUX, PIN>(eos_of<T, MULTI, SG>(a.s, idp), d, Sp, W, delta, F2);
+              if (err2) report(a.err, err2, -1, where + 2);
+#pragma unroll
+              for (int c = 0; c < 5; c++) {
+                FL[0][c] = d == 0 ? F2[c] : FL[0][c];
+                FL[1][c] = d == 1 ? F2[c] : FL[1][c];
+                FL[2][c] = d == 2 ? F2[c] : FL[2][c];
+              }
+            };
+#pragma unroll 1
+            for (int d = 0; d < 3; d++) own_side(d);
           }
         }
-        if (c == 4 && a.visc.fh[0]) {
-          // heat fluxes (HeatDiffusionOperator::AddDiffusionFluxes, after the
-          // viscous ones), energy only, in the same cell order
-          const long long fxi = ((long long)m * g.ny + gj) * (g.nx + 1) + gi;
-          const long long fyi = ((long long)m * (g.ny + 1) + gj) * g.nx + gi;
-          const long long fzi = ((long long)m * g.ny + gj) * g.nx + gi;
-          f = f + a.visc.fh[0][fxi];
-          f = f + a.visc.fh[1][fyi];
-          f = f + a.visc.fh[2][fzi];
-          f = f - a.visc.fh[0][fxi + 1];
-          f = f - a.visc.fh[1][fyi + g.nx];
-          f = f - a.visc.fh[2][fzi + (long long)g.ny * g.nx];
+#pragma unroll
+        for (int c = 0; c < 5; c++) {
+          const T fr = sm.fx[c][row][lane + 1], gr = sm.fy[c][row + 1][lane];
+          if constexpr (sizeof(T) == 8) {
+            // FP64: the reference's order, 0 - Fl A - Gl A - Hl A + Fr A + Gr A + Hr A
+            double f = 0.0;
+            f = f - FL[0][c] * ax;
+            f = f - FL[1][c] * ay;
+            f = f - FL[2][c] * az;
+            f = f + double(fr) * ax;
+            f = f + double(gr) * ay;
+            part[c] = f;
+          } else {
+            // mixed: FP32 accumulation of the flux differences (the difference
+            // of two nearby FP32 fluxes is exact), one conversion per component
+            dxy[c] = (fr - FL[0][c]) * axf + (gr - FL[1][c]) * ayf;
+            hl[c] = FL[2][c];
+          }
         }
-        const double R = f * inv_mvol;
-        if (a.Ro[0]) a.Ro[c][off] = R;
-        Unew[c] = Unew[c] + bdt * R;
       }
-      if (a.Ro[0]) continue;
-      double V[5];
-      e.c2p(Unew, V);
-      const bool clipped = e.clip(V);
-      clipped_local |= clipped ? 1 : 0;
-      if (e.bad(V)) report(a.err, ERR_STATE, (int)((long long)m * g.ny * g.nx + (long long)gj * g.nx + gi), where + 3);
-      if (a.final_stage) {
+      idprev = idp;
 #pragma unroll
-        for (int c = 0; c < 5; c++) a.Vo[c][off] = V[c];
-        if (a.Vfo[0]) {
-#pragma unroll
-          for (int c = 0; c < 5; c++) a.Vfo[c][off] = float(V[c]);
-        }
-        const double ee = e.energy(V[0], V[4]);
-        const double c2 = e.c2(V[0], ee);
-        if (c2 < 0.0) report(a.err, ERR_SOUND, (int)off, where + 4);
-        const double cs = sqrt(c2);
-        const double lx = fabs(V[1]) + cs, ly = fabs(V[2]) + cs, lz = fabs(V[3]) + cs;
-        const double r = smin(dxi / lx, smin(dyj / ly, dzk / lz));
-        dtmin_local = smin(dtmin_local, r);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 5; c++) a.Uo[c][off] = Unew[c];
-        // the next stage's input: clip(C2P(U_new)), as it would recompute it
-#pragma unroll
-        for (int c = 0; c < 5; c++) static_cast<T*>(a.Po[c])[off] = T(V[c]);
-      }
+      for (int c = 0; c < 5; c++) pz[c] = pzn[c];
+    }
+    if (own) {
+      dtmin_local = smin(dtmin_local, smin(dxi / lmax[0], smin(dyj / lmax[1], dzc / lmax[2])));
+      lmax[0] = lmax[1] = lmax[2] = 0.0;
     }
   }
 
   if (a.clipped_out && __syncthreads_or(clipped_local)) {
-    if (tid == 0) atomicOr(a.clipped_out, 1);
+    if (lane == 0 && row == 0) atomicOr(a.clipped_out, 1);
   }
   if (a.final_stage && a.dtmin_bits) {
     double v = dtmin_local;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = smin(v, __shfl_xor_sync(0xffffffffu, v, o));
     __syncthreads();
-    if (tx == 0) sm.red[ty] = v;
+    if (lane == 0 && row < TY) sm.red[row] = v;
     __syncthreads();
-    if (tid == 0) {
+    if (lane == 0 && row == 0) {
       double r = sm.red[0];
       for (int q = 1; q < TY; q++) r = smin(r, sm.red[q]);
       if (r < 1.0e300) atomicMin(a.dtmin_bits, (unsigned long long)__double_as_longlong(r));
