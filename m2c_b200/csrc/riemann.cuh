@@ -81,6 +81,26 @@ struct RPath {
 
 template <typename T> M2C_HD void swap_(T& a, T& b) { T t = a; a = b; b = t; }
 
+// Quotients by one divisor b, each the correctly rounded a / b, for one
+// division and five multiply-adds per quotient. Markstein (IBM Journal of
+// Research and Development 34, 1990): with y = RN(1/b) and q within one unit
+// in the last place of a/b, fma(fma(-b, q, a), y, q) = RN(a/b). The product
+// a y is within 1.5 units, the first correction brings it within one, the
+// second rounds it. Valid where neither a, b nor the quotient comes near the
+// ends of the exponent range: see mid_range.
+struct Divisor {
+  double b, y;
+  M2C_HD explicit Divisor(double d) : b(d), y(1.0 / d) {}
+  M2C_HD double operator()(double a) const {
+    double q = a * y;
+    q = fma(fma(-b, q, a), y, q);
+    return fma(fma(-b, q, a), y, q);
+  }
+};
+// 2^-400 < x < 2^400 (false for NaN): quotients and products of two such
+// numbers, and their remainders down to 2^-110 of them, are normal numbers.
+M2C_HD bool mid_range(double x) { return x > 0x1p-400 && x < 0x1p400; }
+
 struct RiemannSolver {
   RiemannParams P;
   const Eos<double>* eos;  // material table indexed by id
@@ -205,9 +225,9 @@ struct RiemannSolver {
     return false;  // did not reach ps (both of the reference's outcomes fail)
   }
 
-  // Rarefaction_OneStepRK4 (ExactRiemannSolverBase.cpp:1729-1852)
-  M2C_HD bool rk_step(int wave, int id, double rho_0, double u_0, double p_0, double dp, double& rho, double& u,
-                      double& p, double& xi, double& uErr, double& rhoErr) const {
+  // The step for any equation of state and any magnitudes.
+  M2C_HD_OUTLINE bool rk_step_general(int wave, int id, double rho_0, double u_0, double p_0, double dp, double& rho, double& u,
+                      double& p, double& xi, double& uErr, double& rhoErr, double& c_square) const {
     const Eos<double>& e = eos[id];
     dp = -dp;
     double e_0 = e.energy(rho_0, p_0);
@@ -263,9 +283,139 @@ struct RiemannSolver {
     double ee = e.energy(rho, p);
     double c = e.c2(rho, ee);
     if (rho <= 0 || c < 0) return false;
+    c_square = c;
     c = sqrt(c);
     xi = (wave == 1) ? u - c : u + c;
     return true;
+  }
+
+  // Rarefaction_OneStepRK4 (ExactRiemannSolverBase.cpp:1729-1852). c_0_square
+  // is the squared sound speed at (rho_0, p_0); the one at the end of the step
+  // is returned in c_square (the next step's start). A rarefaction is a chain
+  // of up to hundreds of steps that nothing else in the warp can overlap: its
+  // time is this function's instruction count, most of it the step's 56
+  // divisions. For a stiffened gas they share 25 divisors or fewer: one
+  // division each and Divisor's multiply-adds for the rest, the sums kept as
+  // running sums in their order. Same bits as rk_step_general, which takes
+  // the other equations of state and magnitudes.
+  M2C_HD bool rk_step(int wave, int id, double rho_0, double u_0, double p_0, double dp, double c_0_square, double& rho,
+                      double& u, double& p, double& xi, double& uErr, double& rhoErr, double& c_square) const {
+    const Eos<double>& e = eos[id];
+    const double step = dp;
+    const bool fine = e.kind == EOS_SG && mid_range(fabs(dp)) && mid_range(rho_0) && mid_range(c_0_square);
+    if (!fine && (rho_0 <= 0 || c_0_square < 0)) return false;
+    dp = -dp;
+    // squared sound speed at (r, q), as Eos::c2 of Eos::energy; R divides by r.
+    // False where the state or a magnitude is out of range.
+    auto sound = [&](double r, double q, const Divisor& R, double& c2) {
+      const double ei = (q + e.gam_ps) / (e.gam1 * r);
+      const double pr = e.gam1 * r * ei - e.gam_ps;
+      c2 = e.gam1 * ei + R(pr) * e.gam1;
+      return mid_range(r) && mid_range(c2) && (pr == 0.0 || mid_range(fabs(pr)));
+    };
+    if (fine) do {  // left for the general step
+      // stage 0
+      double s1, s2, s3, s4, s5, drho, drho_err, du, du_err;
+      {
+        const Divisor D(c_0_square), C(sqrt(c_0_square)), R(rho_0);
+        s1 = rho_0 + D(0.2 * dp);
+        s2 = rho_0 + D(3. / 40. * dp);
+        s3 = rho_0 + D(3. / 10. * dp);
+        s4 = rho_0 - D(11. / 54. * dp);
+        s5 = rho_0 + D(1631. / 55296. * dp);
+        drho = D(37. / 378.);
+        drho_err = D(2825. / 27648.);
+        du = R(C(37. / 378.));
+        du_err = R(C(2825. / 27648.));
+      }
+      const double p_1 = p_0 + 0.2 * dp;
+      {
+        const Divisor R(s1);
+        double c2;
+        if (!sound(s1, p_1, R, c2)) {
+          if (s1 <= 0 || (mid_range(s1) && c2 < 0)) return false;
+          break;
+        }
+        const Divisor D(c2);
+        s2 = s2 + D(9. / 40. * dp);
+        s3 = s3 - D(9. / 10. * dp);
+        s4 = s4 + D(2.5 * dp);
+        s5 = s5 + D(175. / 512. * dp);
+      }
+      {
+        const Divisor R(s2);
+        double c2;
+        if (!sound(s2, p_1 + 3. / 10. * dp, R, c2)) {
+          if (s2 <= 0 || (mid_range(s2) && c2 < 0)) return false;
+          break;
+        }
+        const Divisor D(c2), C(sqrt(c2));
+        s3 = s3 + D(6. / 5. * dp);
+        s4 = s4 - D(70. / 27. * dp);
+        s5 = s5 + D(575. / 13824. * dp);
+        drho = drho + D(250. / 621.);
+        drho_err = drho_err + D(18575. / 48384.);
+        du = du + R(C(250. / 621.));
+        du_err = du_err + R(C(18575. / 48384.));
+      }
+      {
+        const Divisor R(s3);
+        double c2;
+        if (!sound(s3, p_0 + 3. / 5. * dp, R, c2)) {
+          if (s3 <= 0 || (mid_range(s3) && c2 < 0)) return false;
+          break;
+        }
+        const Divisor D(c2), C(sqrt(c2));
+        s4 = s4 + D(35. / 27. * dp);
+        s5 = s5 + D(44275. / 110592. * dp);
+        drho = drho + D(125. / 594.);
+        drho_err = drho_err + D(13525. / 55296.);
+        du = du + R(C(125. / 594.));
+        du_err = du_err + R(C(13525. / 55296.));
+      }
+      {
+        const Divisor R(s4);
+        double c2;
+        if (!sound(s4, p_0 + dp, R, c2)) {
+          if (s4 <= 0 || (mid_range(s4) && c2 < 0)) return false;
+          break;
+        }
+        const Divisor D(c2), C(sqrt(c2));
+        s5 = s5 + D(253. / 4096. * dp);
+        drho_err = drho_err + D(277. / 14336.);
+        du_err = du_err + R(C(277. / 14336.));
+      }
+      {
+        const Divisor R(s5);
+        double c2;
+        if (!sound(s5, p_0 + 7. / 8. * dp, R, c2)) {
+          if (s5 <= 0 || (mid_range(s5) && c2 < 0)) return false;
+          break;
+        }
+        const Divisor D(c2), C(sqrt(c2));
+        drho = drho + D(512. / 1771.);
+        drho_err = drho_err + D(0.25);
+        du = du + R(C(512. / 1771.));
+        du_err = du_err + R(C(0.25));
+      }
+      drho = drho * dp;
+      drho_err = drho_err * dp;
+      du = du * dp;
+      du_err = du_err * dp;
+      const double r = rho_0 + drho, q = p_0 + dp;
+      double cc;
+      if (!sound(r, q, Divisor(r), cc)) break;  // a failed step leaves its results untouched
+      rhoErr = fabs(drho_err - drho);
+      uErr = fabs(du_err - du);
+      rho = r;
+      p = q;
+      u = (wave == 1) ? u_0 - du : u_0 + du;
+      c_square = cc;
+      cc = sqrt(cc);
+      xi = (wave == 1) ? u - cc : u + cc;
+      return true;
+    } while (false);
+    return rk_step_general(wave, id, rho_0, u_0, p_0, step, rho, u, p, xi, uErr, rhoErr, c_square);
   }
 
   // HugoniotEquation (ExactRiemannSolverBase.h:58-75)
@@ -318,6 +468,7 @@ struct RiemannSolver {
       xi_0 = xi;
       bool done = false;
       double uErr = 0., rhoErr = 0.;
+      double cc_0 = e.c2(rhos_0, e.energy(rhos_0, ps_0)), cc_1 = 0.;  // squared sound speed at the step's ends
       const int moreSteps = 3;
       for (int i = 0; i < P.numSteps_rarefaction * moreSteps; i++) {
         if (fabs(ps_1 - ps) <= pressure_endpoint_tol) {
@@ -327,7 +478,7 @@ struct RiemannSolver {
           done = true;
           break;
         }
-        bool ok = rk_step(wave, id, rhos_0, us_0, ps_0, dp, rhos_1, us_1, ps_1, xi_1, uErr, rhoErr);
+        bool ok = rk_step(wave, id, rhos_0, us_0, ps_0, dp, cc_0, rhos_1, us_1, ps_1, xi_1, uErr, rhoErr, cc_1);
         if (!ok) {
           dp = dp / 2.0;
           continue;
@@ -376,6 +527,7 @@ struct RiemannSolver {
         us_0 = us_1;
         ps_0 = ps_1;
         xi_0 = xi_1;
+        cc_0 = cc_1;
       }
       if (!done) return false;
     } else {  // shock: root of the Hugoniot equation in rhos
@@ -958,8 +1110,9 @@ struct RiemannSolver {
     double r1 = rho, v1 = u, q1 = p, x1;          // end of the step
     const double utol = P.tol_rarefaction * smax(us - u, smax(fabs(us), fabs(u)));
     double errU = 0, errR = 0;
+    double cc_0 = e.c2(rho, e.energy(rho, p)), cc_1 = 0;  // squared sound speed at the step's ends
     for (int i = 0; i < P.numSteps_rarefaction * 5; i++) {
-      if (!rk_step(1, id, r0, v0, q0, dp, r1, v1, q1, x1, errU, errR)) {
+      if (!rk_step(1, id, r0, v0, q0, dp, cc_0, r1, v1, q1, x1, errU, errR, cc_1)) {
         dp /= 2.0;
         continue;
       }
@@ -995,6 +1148,7 @@ struct RiemannSolver {
       v0 = v1;
       q0 = q1;
       x0 = x1;
+      cc_0 = cc_1;
     }
     return false;  // did not reach us (the reference fails either way)
   }

@@ -147,3 +147,8 @@ extern "C" int host_riemann_wall(const m2cg_scheme* s, const m2cg_material* mats
   }
   return 0;
 }
+
+// Quotients of the solver's Divisor.
+extern "C" void host_divisor(int n, const double* a, const double* b, double* q) {
+  for (int i = 0; i < n; i++) q[i] = Divisor(b[i])(a[i]);
+}
