@@ -84,9 +84,14 @@ __device__ __forceinline__ void wall_direction(int mode, int d, int fb, const do
 
 // One thread per one-sided problem (a side of a cut face): the two sides of
 // a face are independent solves, so splitting them doubles the resident
-// warps that hide the FP64 latency of the rarefaction integration (4 CTAs
-// per SM at 128 registers: more resident warps beat the few spills).
-__global__ void __launch_bounds__(128, 4) k_wall_riemann(WallPassArgs a) {
+// warps that hide the FP64 latency of the rarefaction integration. A problem
+// is one chain of up to hundreds of integration steps. CTAS: resident CTAs
+// per SM that the kernel is compiled for. Where the problems fill the chip
+// more than twice, 4 at 128 registers (more resident warps beat the spills);
+// where two CTAs per SM hold them all, 2, whose chains carry no spills (box
+// 96^3 cut by a plane, 5 steps: 13.35 ms with 4, 13.05 with 2).
+template <int CTAS>
+__global__ void __launch_bounds__(128, CTAS) k_wall_riemann(WallPassArgs a) {
   const Grid3& g = a.st.g;
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   RiemannSolver rs;
@@ -273,7 +278,10 @@ m2cg_status walls_stage(Walls* w, cudaStream_t s, StageArgs& a) {
   p.scratch = w->scratch;
   p.nwork = w->nwork;
   p.normal_mode = w->normal_mode;
-  k_wall_riemann<<<w->threads / 128, 128, 0, s>>>(p);
+  if (w->threads <= 2 * 148 * 128)
+    k_wall_riemann<2><<<w->threads / 128, 128, 0, s>>>(p);
+  else
+    k_wall_riemann<4><<<w->threads / 128, 128, 0, s>>>(p);
   if (cudaGetLastError() != cudaSuccess) return M2CG_ERR_CUDA;
   walls_view(w, a);
   return M2CG_OK;
